@@ -63,108 +63,77 @@
 namespace sph {
 
 namespace {
-// Appends slots to a list column.  Plain: four slots at a time (one 16-byte store per four),
-// the group being filled staged in the thread's 16 bytes of shared memory — one store per slot
-// at a computed address, where keeping it in registers took a select per register per slot,
-// and the walk's divergent hit path runs for nearly every candidate a warp tests (build −6%).
-// Interleaved: the window of eight staged the same way (the thread's eight slots NS_MAX_THREADS
-// words apart, so a warp's stores hit 32 banks) and stored as two int4.  Shared memory of a
-// block: SlotWriter<WIN>::kStage int4 per thread.
-template <bool WIN>
-struct SlotWriter;
-
-template <>
-struct SlotWriter<false> {
-    static constexpr int kStage = 1;
-    int* __restrict__ col;
-    int cap;
-    int* buf;  // the thread's four staging slots (shared memory, 16-byte aligned)
-    int cnt = 0;
-    __device__ __forceinline__ SlotWriter(int* c, int cp, int4* stage)
-        : col(c), cap(cp), buf(reinterpret_cast<int*>(stage + threadIdx.x)) {}
-    __device__ __forceinline__ void put(int v) {
-        buf[cnt & 3] = v;
-        cnt++;
-        if ((cnt & 3) == 0 && cnt <= cap)
-            *reinterpret_cast<int4*>(col + ((size_t)(cnt - 4) << 5)) =
-                *reinterpret_cast<const int4*>(buf);
-    }
-    // the last, partial group (its unused slots are never read: count bounds the readers)
-    __device__ __forceinline__ void flush() {
-        if ((cnt & 3) && cnt < cap)
-            *reinterpret_cast<int4*>(col + ((size_t)(cnt & ~3) << 5)) =
-                *reinterpret_cast<const int4*>(buf);
-    }
-};
-
-template <>
-struct SlotWriter<true> {
-    static constexpr int kStage = 2;
-    int* __restrict__ col;
-    int cap;
-    int* buf;  // the thread's eight staging slots, buf[p * NS_MAX_THREADS] (shared memory)
-    int cnt = 0;
-    __device__ __forceinline__ SlotWriter(int* c, int cp, int4* stage)
-        : col(c), cap(cp), buf(reinterpret_cast<int*>(stage) + threadIdx.x) {}
-    // entry e of a window goes to chunk e mod 2, component e / 2
-    __device__ __forceinline__ void put(int v) {
-        const int e = cnt & 7;
-        buf[(((e & 1) << 2) | (e >> 1)) * NS_MAX_THREADS] = v;
-        cnt++;
-        if ((cnt & 7) == 0 && cnt <= cap) store(cnt - 8, 2);
-    }
-    // the last, partial window: its chunks that hold entries (chunk a holds entry a first);
-    // cap is a multiple of 16, so the window fits
-    __device__ __forceinline__ void flush() {
-        const int r = cnt & 7;
-        if (r && cnt < cap) store(cnt & ~7, r > 1 ? 2 : 1);
-    }
-    __device__ __forceinline__ void store(int e0, int chunks) {
-        for (int a = 0; a < chunks; a++) {
-            const int* w = buf + 4 * a * NS_MAX_THREADS;
-            *reinterpret_cast<int4*>(col + ((size_t)(e0 + 4 * a) << 5)) =
-                make_int4(w[0], w[NS_MAX_THREADS], w[2 * NS_MAX_THREADS], w[3 * NS_MAX_THREADS]);
-        }
-    }
-};
-
 // List modes of the one-lane passes (template LIST): no list (cell walks), a list of plain
 // windows, or one of interleaved windows (KParams::list_win).  The mode is a template
 // parameter: a runtime choice between the two loops cost pass 2 1%.
 enum { LIST_NONE = 0, LIST_PLAIN = 1, LIST_WIN = 2 };
 
-// Neighbours of i (r2 < kh2) with their records R[2j], R[2j+1]: from the list (one record
-// load per listed pair, the next slot loaded one pair ahead; pairs in the skin beyond the
-// support radius are skipped), or by walking the cells over X[XSTRIDE * j] when i overflowed
-// the list.  f(j, a, b, dx, dy, dz, r2).  (Skipping the gathers of slots in the skin with a
-// pass-1 hit mask cost pass 2 more in instructions than it saved in sectors.)
-template <class P, int LIST, int XSTRIDE, class F>
+// Whether the passes take a particle's listed neighbours two at a time in two-lane FP32
+// instructions (fluid_two): FP32 pair arithmetic with plain sums.
+template <class P>
+constexpr bool kPairTwo = std::is_same<typename P::T, float>::value && !P::kComp;
+
+// Listed neighbours of a fluid particle, a chunk of four at a time: the four record gathers are
+// issued together and the pairs evaluated without a branch, in list order.
+template <class P, bool WIN, class Acc>
+__device__ __forceinline__ void visit_fluid(const KParamsT<float>& k, const NbrList& nl,
+                                            const float4* __restrict__ R, int t, int cnt,
+                                            Acc& acc) {
+    for_each_chunk<WIN>(nl.idx + nbr_col(nl, t), cnt, 0, 1, [&](const int4& q) {
+        const int e[4] = {q.x, q.y, q.z, q.w};
+        float4 a[4], v[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) ld_rec(R, P::kCodes ? slot_index(e[c]) : e[c], a[c], v[c]);
+#pragma unroll
+        for (int c = 0; c < 4; c += 2)
+            acc.fluid_two(k, a[c], v[c], P::kCodes ? slot_code(e[c]) : 0u, a[c + 1], v[c + 1],
+                          P::kCodes ? slot_code(e[c + 1]) : 0u);
+    });
+}
+
+// Neighbours of slot i (work position t; r2 < kh2) with their records R[2j], R[2j+1]: from the list (pairs in the skin
+// beyond the support radius are skipped), or by walking the cells over X[XSTRIDE * j] when i
+// overflowed the list.  f(j, a, b, dx, dy, dz, r2); with FAST and kPairTwo the list goes through
+// acc.fluid_two instead (a fluid particle).
+template <class P, int LIST, int XSTRIDE, class Acc, class F>
 __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
                                               const int* __restrict__ cs,
                                               const unsigned* __restrict__ keys,
                                               const NbrList& nl,
                                               const vec4_t<typename P::T>* __restrict__ X,
-                                              const vec4_t<typename P::T>* __restrict__ R, int i,
-                                              const vec4_t<typename P::T>& pi, F&& f) {
+                                              const vec4_t<typename P::T>* __restrict__ R, int t,
+                                              int i, Acc& acc, F&& f) {
     using T = typename P::T;
     using V = vec4_t<T>;
     if constexpr (LIST != LIST_NONE) {
-        const int cnt = __ldg(nl.count + i);
+        const int cnt = __ldg(nl.count + t);
         if (cnt <= nl.cap) {
+            if constexpr (kPairTwo<P>) {
+                if (acc.fi) {
+                    visit_fluid<P, LIST == LIST_WIN>(k, nl, R, t, cnt, acc);
+                    return;
+                }
+            }
             auto one = [&](int e) {
                 const int j = P::kCodes ? slot_index(e) : e;
                 V a, b;
                 ld_rec(R, j, a, b);
                 T dx, dy, dz;
-                rel_pos<P>(k, pi, a, P::kCodes ? slot_code(e) : 0u, dx, dy, dz);
+                rel_pos<P>(k, acc.pi, a, P::kCodes ? slot_code(e) : 0u, dx, dy, dz);
                 const T r2 = dist2(dx, dy, dz);
                 if (r2 < k.kh2) f(j, a, b, dx, dy, dz, r2);
             };
-            for_each_slot<LIST == LIST_WIN>(nl.idx + nbr_col(nl, i), cnt, 0, 1, one);
+            for_each_chunk<LIST == LIST_WIN>(nl.idx + nbr_col(nl, t), cnt, 0, 1,
+                                             [&](const int4& q) {
+                one(q.x);
+                one(q.y);
+                one(q.z);
+                one(q.w);
+            });
             return;
         }
     }
-    walk_pairs<P, XSTRIDE>(k, cs, keys, X, i, pi, k.kh2,
+    walk_pairs<P, XSTRIDE>(k, cs, keys, X, i, acc.pi, k.kh2,
                            [&](int j, unsigned, const V&, T dx, T dy, T dz, T r2) {
         V a, b;
         ld_rec(R, j, a, b);
@@ -181,8 +150,9 @@ __device__ __forceinline__ void nbr_build_one(const KParamsT<typename P::T>& k,
                                               const vec4_t<typename P::T>* __restrict__ X,
                                               const unsigned* __restrict__ keys,
                                               const int* __restrict__ cs, const NbrList& nl,
-                                              int walls_all, unsigned* err, int4* stage, int i) {
+                                              int walls_all, unsigned* err, int4* stage, int t) {
     using T = typename P::T;
+    const int i = work_slot(nl, t);
     T cut2 = nl.cut2 ? (T)__ldg(nl.cut2) : k.kh2_list;
     if (nl.iw) {
         // per-instance decisions: the particles of the instances that rebuild, each at its
@@ -207,11 +177,11 @@ __device__ __forceinline__ void nbr_build_one(const KParamsT<typename P::T>& k,
                     any = any || __ldg(nl.fluid_cells + row + x) != 0;
             }
         if (!any) {
-            nl.count[i] = 0;
+            nl.count[t] = 0;
             return;
         }
     }
-    SlotWriter<WIN> w(nl.idx + nbr_col(nl, i), nl.cap, stage);
+    SlotWriter<WIN> w(nl.idx + nbr_col(nl, t), nl.cap, stage);
     if constexpr (P::kCodes) {
         // i's offsets moved into each run's anchor frame once per run instead of decoding the
         // code for every candidate.  That rounds differently from the passes' decode, so the
@@ -259,8 +229,8 @@ __device__ __forceinline__ void nbr_build_one(const KParamsT<typename P::T>& k,
             }, win);
         }
     }
-    w.flush();
-    nl.count[i] = w.cnt;
+    w.flush(pad_slot<P>(k.n));
+    nl.count[t] = w.cnt;
     raise_flags(err, w.cnt > nl.cap ? SPH_FLAG_NEIGHBOR_OVERFLOW : 0u);
 }
 
@@ -268,11 +238,16 @@ template <class P, bool GS, bool WIN>
 __global__ void __launch_bounds__(NS_MAX_THREADS)
 k_nbr_build(KParamsT<typename P::T> k, const vec4_t<typename P::T>* __restrict__ X,
             const unsigned* __restrict__ keys, const int* __restrict__ cs, NbrList nl,
-            int walls_all, unsigned* err, const unsigned* gate) {
+            vec4_t<typename P::T>* rec, vec4_t<typename P::T>* nrec, int walls_all, unsigned* err,
+            const unsigned* gate) {
     __shared__ int4 s_stage[SlotWriter<WIN>::kStage * NS_MAX_THREADS];
     if (gated_off(gate)) return;
     int4* stage = s_stage;
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i0 == 0) {
+        pad_record<typename P::T>(rec, k.n);
+        pad_record<typename P::T>(nrec, k.n);
+    }
     if constexpr (GS) {
         for (int i = i0; i < k.n; i += gridDim.x * blockDim.x)
             nbr_build_one<P, WIN>(k, X, keys, cs, nl, walls_all, err, stage, i);
@@ -288,20 +263,25 @@ __device__ __forceinline__ void pass1_one(const KParamsT<typename P::T>& k,
                                           const int* __restrict__ cs, const NbrList& nl,
                                           const Pass1OutT<typename P::T>& out,
                                           float* __restrict__ rhop_sum, float* __restrict__ w_sum,
-                                          int i) {
+                                          int t) {
     using T = typename P::T;
     using V = vec4_t<T>;
+    const int i = work_slot(nl, t);
     Pass1Acc<P> acc;
     acc.load(in.rec, i);
-    visit_records<P, LIST, 1>(k, cs, keys, nl, in.xyz, in.rec, i, acc.pi,
+    visit_records<P, LIST, 1>(k, cs, keys, nl, in.xyz, in.rec, t, i, acc,
                               [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
         acc.pair(k, aj, vj, dx, dy, dz, r2);
     });
     acc.template finish<WRITE_SUMS>(k, out, rhop_sum, w_sum, i);
 }
 
+// Registers of pass 1: room for the four records of a chunk in flight.
+template <class P>
+constexpr int kPass1Regs = std::is_same<typename P::T, double>::value ? 96 : 72;
+
 template <class P, bool WRITE_SUMS, int LIST, bool GS>
-__global__ void __launch_bounds__(NS_MAX_THREADS)
+__global__ void __maxnreg__(kPass1Regs<P>)
 k_pass1(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         const unsigned* __restrict__ keys, const int* __restrict__ cs, NbrList nl,
         Pass1OutT<typename P::T> out, float* __restrict__ rhop_sum, float* __restrict__ w_sum) {
@@ -314,7 +294,7 @@ k_pass1(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
     }
 }
 template <class P, int MODE, int LIST>
-__device__ __forceinline__ void pass2_one(const KParamsT<typename P::T>& k, int i,
+__device__ __forceinline__ void pass2_one(const KParamsT<typename P::T>& k, int t,
                                           const ParticleSetT<typename P::T>& in,
                                           const unsigned* __restrict__ keys,
                                           const int* __restrict__ cs, const NbrList& nl,
@@ -325,10 +305,11 @@ __device__ __forceinline__ void pass2_one(const KParamsT<typename P::T>& k, int 
                                           DispBox& box, unsigned* disp) {
     using T = typename P::T;
     using V = vec4_t<T>;
+    const int i = work_slot(nl, t);
     Pass2Acc<P, MODE> acc;
     acc.load(k, p1, i, wall_rates);
     if (acc.active)
-        visit_records<P, LIST, 2>(k, cs, keys, nl, p1.nrec, p1.nrec, i, acc.pi,
+        visit_records<P, LIST, 2>(k, cs, keys, nl, p1.nrec, p1.nrec, t, i, acc,
                                   [&](int j, const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
             acc.pair(k, p1, j, aj, vj, dx, dy, dz, r2);
         });
@@ -361,13 +342,11 @@ k_pass2(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
     reduce_disp(k, box, disp, s_box, s_inst);
 }
 
-// The same kernel held to CAP registers (one particle per thread).  The FP32 step kernel (and
-// the one of mixed precision on FP32 positions) runs in 40: six 256-thread blocks per SM
-// instead of the five of its spill-free 48, for 40 bytes of spill
-// (0.610 against 0.634 ms at 4.96M particles; before the pair approximations were taken in
-// their flush-to-zero forms, with more instructions per pair to hide the gathers, the two
-// measured the same).  The mixed-precision kernel on cell-local offsets runs in 56 (nine
-// 128-thread blocks instead of eight).
+// The same kernel held to CAP registers (one particle per thread): room for a chunk's four records
+// in flight with the most warps that leaves.  At 133,968 particles (linear EOS) 80 registers run
+// in 29 us, 64 in 35, 48 in 49, against 44 for one gather at a time in 40; at 380,000 80 run in
+// 45 us, 96 in 55.  The kernel on cell-local offsets keeps 72 (380,000 particles: 77 us, 79 at 80,
+// 83 at 64).
 template <class P, int MODE, int LIST, bool GS, int CAP>
 __global__ void __maxnreg__(CAP)
 k_pass2_cap(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
@@ -445,7 +424,7 @@ void pass2_launch_gs(const KParamsT<typename P::T>& k, const ParticleSetT<typena
     auto with_list = [&](auto mode) {
         constexpr int L = decltype(mode)::value;
         if constexpr (MODE != MODE_RATES && !GS && (P::kId == SPH_PREC_FP32 || P::kMixed)) {
-            constexpr int cap = P::kCodes ? 56 : 40;
+            constexpr int cap = P::kCodes ? 72 : 80;
             k_pass2_cap<P, MODE, L, GS, cap><<<b, k.threads, 0, s>>>(
                 k, in, keys, cs, *nl, p1, rho_dt, vel_dt, wall_rates, out, out_hash, err, disp);
         } else {
@@ -492,23 +471,23 @@ int nbr_capacity_for(const sph_params& p, double skin) {
 template <class P>
 cudaError_t launch_nbr_build(const KParamsT<typename P::T>& k,
                              const ParticleSetT<typename P::T>& in, const unsigned* keys,
-                             const int* cs, const NbrList& nl, int walls_all, unsigned* err,
-                             cudaStream_t s, const unsigned* gate) {
+                             const int* cs, const NbrList& nl, vec4_t<typename P::T>* nrec,
+                             int walls_all, unsigned* err, cudaStream_t s, const unsigned* gate) {
     if (k.n <= 0) return cudaSuccess;
     const dim3 g = ns_grid(k);
     if (k.ppt > 1) {
         if (k.list_win)
-            k_nbr_build<P, true, true><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl,
+            k_nbr_build<P, true, true><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl, in.rec, nrec,
                                                                 walls_all, err, gate);
         else
-            k_nbr_build<P, true, false><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl,
+            k_nbr_build<P, true, false><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl, in.rec, nrec,
                                                                  walls_all, err, gate);
     } else {
         if (k.list_win)
-            k_nbr_build<P, false, true><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl,
+            k_nbr_build<P, false, true><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl, in.rec, nrec,
                                                                  walls_all, err, gate);
         else
-            k_nbr_build<P, false, false><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl,
+            k_nbr_build<P, false, false><<<g, k.threads, 0, s>>>(k, in.xyz, keys, cs, nl, in.rec, nrec,
                                                                   walls_all, err, gate);
     }
     return cudaGetLastError();
@@ -559,8 +538,9 @@ cudaError_t launch_pass2_step(const KParamsT<typename P::T>& k, HalfStep half,
 
 #define SPH_NS_INSTANTIATE(P)                                                                  \
     template cudaError_t launch_nbr_build<P>(const KParamsT<P::T>&, const ParticleSetT<P::T>&, \
-                                             const unsigned*, const int*, const NbrList&, int, \
-                                             unsigned*, cudaStream_t, const unsigned*);        \
+                                             const unsigned*, const int*, const NbrList&,      \
+                                             vec4_t<P::T>*, int, unsigned*, cudaStream_t,      \
+                                             const unsigned*);                                 \
     template cudaError_t launch_pass1<P>(const KParamsT<P::T>&, const ParticleSetT<P::T>&,     \
                                          const unsigned*, const int*, const NbrList*,          \
                                          const Pass1OutT<P::T>&, float*, float*, cudaStream_t);\

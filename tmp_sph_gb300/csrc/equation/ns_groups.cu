@@ -77,12 +77,12 @@ __device__ __forceinline__ void visit_group(const KParamsT<typename P::T>& k,
                                             const unsigned* __restrict__ keys,
                                             const NbrList& nl,
                                             const vec4_t<typename P::T>* __restrict__ X,
-                                            const vec4_t<typename P::T>* __restrict__ R, int i,
+                                            const vec4_t<typename P::T>* __restrict__ R, int t, int i,
                                             const vec4_t<typename P::T>& pi, F&& f) {
     using T = typename P::T;
     using V = vec4_t<T>;
     const int s = sub_lane<G>();
-    const int cnt = __ldg(nl.count + i);
+    const int cnt = __ldg(nl.count + t);
     if (cnt <= nl.cap) {
         auto one = [&](int e) {
             const int j = P::kCodes ? slot_index(e) : e;
@@ -95,10 +95,16 @@ __device__ __forceinline__ void visit_group(const KParamsT<typename P::T>& k,
         };
         // this lane's chunks s, s + G, ... (each pair of lanes gathers two consecutive entries
         // per step)
+        auto four = [&](const int4& q) {
+            one(q.x);
+            one(q.y);
+            one(q.z);
+            one(q.w);
+        };
         if (k.list_win)
-            for_each_slot<true>(nl.idx + nbr_col(nl, i), cnt, s, G, one);
+            for_each_chunk<true>(nl.idx + nbr_col(nl, t), cnt, s, G, four);
         else
-            for_each_slot<false>(nl.idx + nbr_col(nl, i), cnt, s, G, one);
+            for_each_chunk<false>(nl.idx + nbr_col(nl, t), cnt, s, G, four);
         return;
     }
     // the cells one by one (each a contiguous slot range), G candidates per step
@@ -153,11 +159,12 @@ k_pass1_g(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
 #pragma unroll 1
     for (int r = 0; r < G; r++) {
         const int loc = r * (nt / G) + (int)threadIdx.x / G;
-        const int i = base + loc;
+        const int t = base + loc;
         Pass1Acc<P> acc;
-        if (i < k.n) {
+        if (t < k.n) {
+            const int i = work_slot(nl, t);
             acc.load(in.rec, i);
-            visit_group<P, G, 1>(k, cs, keys, nl, in.xyz, in.rec, i, acc.pi,
+            visit_group<P, G, 1>(k, cs, keys, nl, in.xyz, in.rec, t, i, acc.pi,
                                  [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
                 acc.pair(k, aj, vj, dx, dy, dz, r2);
             });
@@ -172,8 +179,9 @@ k_pass1_g(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         }
     }
     __syncthreads();
-    const int i = base + (int)threadIdx.x;
-    if (i < k.n) {
+    const int t = base + (int)threadIdx.x;
+    if (t < k.n) {
+        const int i = work_slot(nl, t);
         Pass1Acc<P> acc;
         acc.load(in.rec, i);
         acc.dofv = sum_of<T, P::kComp>(s_sum[0][threadIdx.x]);

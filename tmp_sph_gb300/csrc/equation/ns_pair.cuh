@@ -27,6 +27,12 @@ __device__ __forceinline__ unsigned slot_code(int e) { return (unsigned)e >> COD
 __device__ __forceinline__ int make_slot(int j, unsigned code) {
     return (int)((unsigned)j | (code << CODE_SHIFT));
 }
+// Padding slot of a list of n particles: record n, which the build puts far outside any support
+// radius (pad_record), so evaluating it adds nothing.
+template <class P>
+__device__ __forceinline__ int pad_slot(int n) {
+    return P::kCodes ? make_slot(n, (1u << 4) | (1u << 2) | 1u) : n;
+}
 // Code of a neighbour cell (xj, yj, zj) seen from cell (xi, yi, zi), both within one walk:
 // the difference of their anchors (anchor_of) in anchor steps, each in {-1, 0, 1}, two bits
 // per axis, (dz+1) << 4 | (dy+1) << 2 | (dx+1).
@@ -43,12 +49,16 @@ __device__ __forceinline__ unsigned cell_code(const KP& k, int xi, int yi, int z
            (anchor_step(yj, anchor_of(yi, r), r) << 2) | anchor_step(xj, anchor_of(xi, r), r);
 }
 
-// Column of particle i in the warp-interleaved list: slots 4g .. 4g+3 of i are the int4 at
+// Slot of work position t.
+__device__ __forceinline__ int work_slot(const NbrList& nl, int t) {
+    return nl.order ? __ldg(nl.order + t) : t;
+}
+// Column of work position t in the warp-interleaved list: slots 4g .. 4g+3 of it are the int4 at
 // col + 32 * 4g (col = the warp's block + 4 * lane).  The 32 particles of a warp share one block
 // of cap x 32 slots, so a warp reading slot group g of all its lanes touches four consecutive
 // lines (512 bytes) with one 16-byte load per lane, and the build stores four slots at a time.
-__device__ __forceinline__ size_t nbr_col(const NbrList& nl, int i) {
-    return (size_t)(i >> 5) * ((size_t)nl.cap << 5) + ((size_t)(i & 31) << 2);
+__device__ __forceinline__ size_t nbr_col(const NbrList& nl, int t) {
+    return (size_t)(t >> 5) * ((size_t)nl.cap << 5) + ((size_t)(t & 31) << 2);
 }
 
 // Four list slots.  The slots stream past once per pass, so they are read without allocating
@@ -76,28 +86,105 @@ __device__ __forceinline__ int chunk_first(int c) {
     return WIN ? c + 6 * (c >> 1) : c << 2;
 }
 
-// one(slot) for the entries of a column (cnt <= cap of them) in chunks c0, c0 + dc, ... (the
-// one-lane passes: c0 = 0, dc = 1; lane s of a group of G: c0 = s, dc = G), four to an int4,
-// the next chunk loaded one chunk ahead (four record gathers in flight per thread).  Chunk
-// firsts grow with c, so the first chunk past the count ends the column.
+// four(slots) for the chunks c0, c0 + dc, ... of a column of cnt <= cap entries (the one-lane
+// passes: c0 = 0, dc = 1; lane s of a group of G: c0 = s, dc = G), the next chunk loaded one
+// ahead.  The build fills the last chunk up with the padding slot (pad_slot), so a chunk is always
+// four slots and the callers carry no count guards.  Chunk firsts grow with c, so the first chunk
+// past the count ends the column.
 template <bool WIN, class F>
-__device__ __forceinline__ void for_each_slot(const int* __restrict__ col, int cnt, int c0,
-                                              int dc, F&& one) {
-    constexpr int st = WIN ? 2 : 1;
-    int c = c0, e = chunk_first<WIN>(c0);
-    int4 q = e < cnt ? ld_slots(col + ((size_t)c << 7)) : make_int4(0, 0, 0, 0);
+__device__ __forceinline__ void for_each_chunk(const int* __restrict__ col, int cnt, int c0,
+                                               int dc, F&& four) {
+    int c = c0;
+    bool more = chunk_first<WIN>(c) < cnt;
+    int4 q = more ? ld_slots(col + ((size_t)c << 7)) : make_int4(0, 0, 0, 0);
 #pragma unroll 1
-    while (e < cnt) {
-        const int cn = c + dc, en = chunk_first<WIN>(cn);
-        const int4 qn = en < cnt ? ld_slots(col + ((size_t)cn << 7)) : q;
-        one(q.x);
-        if (e + st < cnt) one(q.y);
-        if (e + 2 * st < cnt) one(q.z);
-        if (e + 3 * st < cnt) one(q.w);
+    while (more) {
+        c += dc;
+        more = chunk_first<WIN>(c) < cnt;
+        const int4 qn = more ? ld_slots(col + ((size_t)c << 7)) : q;
+        four(q);
         q = qn;
-        c = cn;
-        e = en;
     }
+}
+
+// Appends slots to a list column.  Plain: four slots at a time (one 16-byte store per four),
+// the group being filled staged in the thread's 16 bytes of shared memory — one store per slot
+// at a computed address, where keeping it in registers took a select per register per slot,
+// and the walk's divergent hit path runs for nearly every candidate a warp tests (build −6%).
+// Interleaved: the window of eight staged the same way (the thread's eight slots NS_MAX_THREADS
+// words apart, so a warp's stores hit 32 banks) and stored as two int4.  Shared memory of a
+// block: SlotWriter<WIN>::kStage int4 per thread.
+template <bool WIN>
+struct SlotWriter;
+
+template <>
+struct SlotWriter<false> {
+    static constexpr int kStage = 1;
+    int* __restrict__ col;
+    int cap;
+    int* buf;  // the thread's four staging slots (shared memory, 16-byte aligned)
+    int cnt = 0;
+    __device__ __forceinline__ SlotWriter(int* c, int cp, int4* stage)
+        : col(c), cap(cp), buf(reinterpret_cast<int*>(stage + threadIdx.x)) {}
+    __device__ __forceinline__ void put(int v) {
+        buf[cnt & 3] = v;
+        cnt++;
+        if ((cnt & 3) == 0 && cnt <= cap)
+            *reinterpret_cast<int4*>(col + ((size_t)(cnt - 4) << 5)) =
+                *reinterpret_cast<const int4*>(buf);
+    }
+    // the last, partial group, filled up with `pad`
+    __device__ __forceinline__ void flush(int pad) {
+        if ((cnt & 3) && cnt < cap) {
+            for (int e = cnt & 3; e < 4; e++) buf[e] = pad;
+            *reinterpret_cast<int4*>(col + ((size_t)(cnt & ~3) << 5)) =
+                *reinterpret_cast<const int4*>(buf);
+        }
+    }
+};
+
+template <>
+struct SlotWriter<true> {
+    static constexpr int kStage = 2;
+    int* __restrict__ col;
+    int cap;
+    int* buf;  // the thread's eight staging slots, buf[p * NS_MAX_THREADS] (shared memory)
+    int cnt = 0;
+    __device__ __forceinline__ SlotWriter(int* c, int cp, int4* stage)
+        : col(c), cap(cp), buf(reinterpret_cast<int*>(stage) + threadIdx.x) {}
+    // entry e of a window goes to chunk e mod 2, component e / 2
+    __device__ __forceinline__ void set(int e, int v) {
+        buf[(((e & 1) << 2) | (e >> 1)) * NS_MAX_THREADS] = v;
+    }
+    __device__ __forceinline__ void put(int v) {
+        set(cnt & 7, v);
+        cnt++;
+        if ((cnt & 7) == 0 && cnt <= cap) store(cnt - 8, 2);
+    }
+    // the last, partial window, filled up with `pad`: its chunks that hold entries (chunk a holds
+    // entry a first); cap is a multiple of 16, so the window fits
+    __device__ __forceinline__ void flush(int pad) {
+        const int r = cnt & 7;
+        if (r && cnt < cap) {
+            for (int e = r; e < 8; e++) set(e, pad);
+            store(cnt & ~7, r > 1 ? 2 : 1);
+        }
+    }
+    __device__ __forceinline__ void store(int e0, int chunks) {
+        for (int a = 0; a < chunks; a++) {
+            const int* w = buf + 4 * a * NS_MAX_THREADS;
+            *reinterpret_cast<int4*>(col + ((size_t)(e0 + 4 * a) << 5)) =
+                make_int4(w[0], w[NS_MAX_THREADS], w[2 * NS_MAX_THREADS], w[3 * NS_MAX_THREADS]);
+        }
+    }
+};
+
+// The record of the lists' padding slot, slot n of the arrays the passes gather from: farther than
+// any support radius from everything (its squared distance stays finite in FP32).
+template <class T>
+__device__ __forceinline__ void pad_record(vec4_t<T>* R, int n) {
+    R[2 * (size_t)n] = make4<T>(T(1e18), T(1e18), T(1e18), T(0));
+    R[2 * (size_t)n + 1] = make4<T>(T(0), T(0), T(0), T(-1));
 }
 
 // Squared distance with an explicit rounding sequence, so the in-range test gives the same
@@ -337,6 +424,36 @@ __device__ __forceinline__ void sub2_rn(double ax, double ay, double bx, double 
     dy = sub_rn(ay, by);
 }
 
+// Two FP32 values in one 64-bit register, and the two-lane instructions on them: each lane is
+// rounded as the scalar instruction rounds it, for one issue slot instead of two.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(F2 x, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 both(float a) { return pack2(a, a); }
+__device__ __forceinline__ F2 mul2_rn(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2_rn(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2_rn(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
 // Relative position r = x_i - x_j of a pair: from positions in the simulation's frame, or
 // (cell codes) from the offsets from their anchor cells and j's anchor relative to i's
 // (anchor steps of reach cells).
@@ -361,6 +478,23 @@ __device__ __forceinline__ void rel_pos(const KParamsT<typename P::T>& k, const 
         (void)code;
         sub2_rn(pi.x, pi.y, pj.x, pj.y, dx, dy);
         dz = sub_rn(pi.z, pj.z);
+    }
+}
+
+// rel_pos, and with it s = s0 - q_j, the fourth component of j's record riding in the two-lane
+// subtraction of the third.
+template <class P>
+__device__ __forceinline__ void rel_pos_s(const KParamsT<float>& k, const float4& pi, float s0,
+                                          const float4& pj, unsigned code, float& dx, float& dy,
+                                          float& dz, float& s) {
+    sub2_rn(pi.x, pi.y, pj.x, pj.y, dx, dy);
+    sub2_rn(pi.z, s0, pj.z, pj.w, dz, s);
+    if constexpr (P::kCodes) {
+        float fx, fy, fz;
+        code_steps(code, fx, fy, fz);
+        dx = fma_rn(-fx, k.reach_cell, dx);
+        dy = fma_rn(-fy, k.reach_cell, dy);
+        dz = fma_rn(-fz, k.reach_cell, dz);
     }
 }
 
@@ -409,6 +543,30 @@ __device__ __forceinline__ T dot_rn(const V& vi, const V& vj, T dx, T dy, T dz) 
     return fma_rn(sub_rn(vi.z, vj.z), dz, fma_rn(uy, dy, mul_rn(ux, dx)));
 }
 
+// s += a b for a pair inside the support radius (r2 < kh2) with a fluid neighbour (rho > 0).
+__device__ __forceinline__ void add_if(float r2, float kh2, float rho, float a, float b,
+                                       float& s) {
+    asm("{.reg .pred p, q;\n\t"
+        "setp.lt.f32 p, %1, %2;\n\t"
+        "setp.gt.and.f32 q, %3, 0f00000000, p;\n\t"
+        "@q fma.rn.f32 %0, %4, %5, %0;}"
+        : "+f"(s)
+        : "f"(r2), "f"(kh2), "f"(rho), "f"(a), "f"(b));
+}
+// sd += w e, (sx, sy, sz) += c (dx, dy, dz) for a pair inside the support radius.
+__device__ __forceinline__ void add_if(float r2, float kh2, float w, float e, float c, float dx,
+                                       float dy, float dz, float& sd, float& sx, float& sy,
+                                       float& sz) {
+    asm("{.reg .pred p;\n\t"
+        "setp.lt.f32 p, %4, %5;\n\t"
+        "@p fma.rn.f32 %0, %6, %7, %0;\n\t"
+        "@p fma.rn.f32 %1, %8, %9, %1;\n\t"
+        "@p fma.rn.f32 %2, %8, %10, %2;\n\t"
+        "@p fma.rn.f32 %3, %8, %11, %3;}"
+        : "+f"(sd), "+f"(sx), "+f"(sy), "+f"(sz)
+        : "f"(r2), "f"(kh2), "f"(w), "f"(e), "f"(c), "f"(dx), "f"(dy), "f"(dz));
+}
+
 // Pass-1 state of one particle: its own record and the three neighbour sums.
 template <class P>
 struct Pass1Acc {
@@ -440,6 +598,27 @@ struct Pass1Acc {
             const T vdotr = dot_rn(vi, vj, dx, dy, dz);
             dofv.add_prod(-mul_rn(fr, vdotr), mul_rn(k.mass, pair_rcp(vj.w)));
         }
+    }
+    // Two neighbours of a fluid particle, given by their records: pair() on each, in order, with
+    // the arithmetic after the pair products in two-lane instructions and the sum taken under a
+    // predicate instead of a branch.
+    __device__ __forceinline__ void fluid_two(const KParamsT<T>& k, const V& aj, const V& vj,
+                                              unsigned cj, const V& al, const V& vl, unsigned cl) {
+        T ax, ay, az, bx, by, bz;
+        rel_pos<P>(k, pi, aj, cj, ax, ay, az);
+        rel_pos<P>(k, pi, al, cl, bx, by, bz);
+        const T r2a = dist2(ax, ay, az), r2b = dist2(bx, by, bz);
+        const F2 rr = pack2(pair_sqrt(r2a), pair_sqrt(r2b));
+        const F2 t = fma2_rn(F2{k.m_half2}, mul2_rn(rr, F2{k.inv_h2}), F2{k.one2});
+        const F2 fr = mul2_rn(mul2_rn(F2{k.c_fr2}, mul2_rn(t, t)), t);
+        const F2 vdotr = pack2(dot_rn(vi, vj, ax, ay, az), dot_rn(vi, vl, bx, by, bz));
+        const F2 u = mul2_rn(fr, vdotr);
+        const F2 m = mul2_rn(both(k.mass), pack2(pair_rcp(vj.w), pair_rcp(vl.w)));
+        float ua, ub, ma, mb;
+        unpack2(u, ua, ub);
+        unpack2(m, ma, mb);
+        add_if(r2a, k.kh2, vj.w, -ua, ma, dofv.s);
+        add_if(r2b, k.kh2, vl.w, -ub, mb, dofv.s);
     }
     template <bool WRITE_SUMS>
     __device__ __forceinline__ void finish(const KParamsT<T>& k, const Pass1OutT<T>& out,
@@ -525,6 +704,36 @@ struct Pass2Acc {
         sx.add_prod(c, dx);
         sy.add_prod(c, dy);
         sz.add_prod(c, dz);
+    }
+    // Two neighbours of a fluid particle, given by their records: pair() on each, in order, with
+    // the arithmetic after the pair products in two-lane instructions and the sums taken under a
+    // predicate instead of a branch.
+    __device__ __forceinline__ void fluid_two(const KParamsT<T>& k, const V& aj, const V& vj,
+                                              unsigned cj, const V& al, const V& vl, unsigned cl) {
+        T ax, ay, az, sa, bx, by, bz, sb;
+        rel_pos_s<P>(k, pi, -presi, aj, cj, ax, ay, az, sa);
+        rel_pos_s<P>(k, pi, -presi, al, cl, bx, by, bz, sb);
+        const T r2a = dist2(ax, ay, az), r2b = dist2(bx, by, bz);
+        const F2 r2 = pack2(r2a, r2b);
+        const T rja = dabs(vj.w), rjb = dabs(vl.w);
+        const F2 rr = pack2(pair_sqrt(r2a), pair_sqrt(r2b));
+        const F2 t = fma2_rn(F2{k.m_half_inv_h2}, rr, F2{k.one2});
+        const F2 w = mul2_rn(mul2_rn(mul2_rn(F2{k.c_fr_mass2}, mul2_rn(t, t)), t),
+                             pack2(pair_rcp(rja), pair_rcp(rjb)));
+        const F2 vdotr = pack2(dot_rn(vi, vj, ax, ay, az), dot_rn(vi, vl, bx, by, bz));
+        float ea, eb;
+        unpack2(add2_rn(r2, F2{k.eta2_2}), ea, eb);
+        const F2 inv = pack2(pair_rcp(ea), pair_rcp(eb));
+        const F2 dr = pack2(sub_rn(rhoi, rja), sub_rn(rhoi, rjb));
+        const F2 diff = mul2_rn(mul2_rn(mul2_rn(dr, F2{k.delta_h_cs2}), r2), inv);
+        unpack2(fma2_rn(both(rhoi), vdotr, diff), ea, eb);
+        float va, vb, wa, wb;
+        unpack2(fma2_rn(mul2_rn(F2{k.visc2}, vdotr), inv, both(damp_i)), va, vb);
+        unpack2(w, wa, wb);
+        const T ca = mul_rn(wa, fluid_rec(vj.w) ? add_rn(sa, va) : sa);
+        const T cb = mul_rn(wb, fluid_rec(vl.w) ? add_rn(sb, vb) : sb);
+        add_if(r2a, k.kh2, wa, ea, ca, ax, ay, az, sd.s, sx.s, sy.s, sz.s);
+        add_if(r2b, k.kh2, wb, eb, cb, bx, by, bz, sd.s, sx.s, sy.s, sz.s);
     }
 };
 

@@ -87,6 +87,10 @@ struct KParamsT {
     // 1: batched instances keep a displacement box each and rebuild their lists on their own
     // decisions (IW_* words below); 0: one box and one decision for all particles
     int inst_boxes;
+    // FP32 constants of the pair arithmetic twice over, as operands of two-lane instructions
+    // (unused by the FP64 kernels)
+    unsigned long long inv_h2, m_half_inv_h2, one2, m_half2, c_fr2, c_fr_mass2, eta2_2,
+        delta_h_cs2, visc2;
 };
 using KParams = KParamsT<float>;
 

@@ -116,7 +116,7 @@ inline bool prec_has_codes(int prec) {
 // Mixed precision (kMixed): xm holds the FP64 position and rho - rho0, txm the predictor's save
 // of it (tpos is unused); x, y, z in rec and xyz are the offsets from the origin of the
 // particle's anchor cell at the last list build (kCodes) or the FP64 position rounded to FP32
-// (PrecMixA).
+// (PrecMixA).  rec has one record more than the capacity: the lists' padding slot (record n).
 template <class T>
 struct ParticleSetT {
     vec4_t<T>* rec = nullptr;
@@ -169,13 +169,19 @@ struct NbrList {
     // every particle is rebuilt at cut2
     const unsigned* iw = nullptr;
     const int* inst = nullptr;
+    // work order: thread t of the list kernels takes slot order[t] (all fluid slots first), and
+    // the list columns and counts are indexed by t; NULL: slot t
+    const int* order = nullptr;
 };
 // List slots per particle: 1.5x the lattice particles within kh (1 + skin), rounded up to 16.
 int nbr_capacity_for(const sph_params& p, double skin = 0.0);
 
 // Neighbour passes (equation/ns.cu), one instantiation per precision policy P.
 // nl == NULL walks the cells in every pass.
-//  build : fills nl for the sorted set (walls keep only fluid neighbours unless walls_all).
+//  build : fills nl for the sorted set (walls keep only fluid neighbours unless walls_all); the
+//          last chunk of four slots of every list is filled up with slot n, and record n of
+//          in.rec and of nrec (the pass-1 records pass 2 gathers) set beyond every support
+//          radius, so the passes read whole chunks.
 //  pass 1: fills a Pass1Out — boundary particles get the extrapolated p and rho, fluid
 //          particles their own p, rho and the velocity divergence.  rhop_sum / w_sum are
 //          written when non-NULL (FP32 only).
@@ -185,8 +191,9 @@ int nbr_capacity_for(const sph_params& p, double skin = 0.0);
 template <class P>
 cudaError_t launch_nbr_build(const KParamsT<typename P::T>& k,
                              const ParticleSetT<typename P::T>& in, const unsigned* sorted_keys,
-                             const int* cell_start, const NbrList& nl, int walls_all,
-                             unsigned* err, cudaStream_t s, const unsigned* gate = nullptr);
+                             const int* cell_start, const NbrList& nl,
+                             vec4_t<typename P::T>* nrec, int walls_all, unsigned* err,
+                             cudaStream_t s, const unsigned* gate = nullptr);
 template <class P>
 cudaError_t launch_pass1(const KParamsT<typename P::T>& k, const ParticleSetT<typename P::T>& in,
                          const unsigned* sorted_keys, const int* cell_start, const NbrList* nl,
@@ -210,6 +217,13 @@ cudaError_t launch_pass2_step(const KParamsT<typename P::T>& k, HalfStep half,
 // Resident-state glue (lib/mesh.cu), one instantiation per precision policy P.
 // perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
 // cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).
+// The work order of the list kernels (NbrList::order) of a cell-sorted set on `grid`: its fluid
+// slots, then the others, each in slot order or (rows) with pairs of rows merged so that
+// consecutive positions hold particles one above the other.  Scratch: rank (n + 1 ints) and
+// tiles (one word per 4096 slots).
+cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int* type,
+                              const unsigned* keys, const int* cs, int* rank, unsigned* tiles,
+                              int* order, cudaStream_t s, const unsigned* gate);
 template <class P>
 cudaError_t launch_gather(const KParamsT<typename P::T>& k, const int* perm,
                           const ParticleSetT<typename P::T>& src, ParticleSetT<typename P::T> dst,

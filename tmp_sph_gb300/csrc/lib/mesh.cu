@@ -427,6 +427,120 @@ __global__ void k_gather(KParamsT<typename P::T> kp, const int* __restrict__ per
     if (with_tmp) dst.tvel[k] = src.tvel[s];
 }
 
+// ---------------------------------------------------------------- work order
+// Fluid slots of each tile of WO_TILE slots, the exclusive scan of those counts (one block), and
+// from it rank[i], the number of fluid slots before slot i (0 <= i <= n).
+constexpr int WO_THREADS = 256;
+constexpr int WO_PER_THREAD = 16;
+constexpr int WO_TILE = WO_THREADS * WO_PER_THREAD;
+
+__global__ void __launch_bounds__(WO_THREADS)
+k_fluid_count(int n, const int* __restrict__ type, unsigned* __restrict__ tiles,
+              const unsigned* gate) {
+    if (gated_off(gate)) return;
+    const long base = (long)blockIdx.x * WO_TILE;
+    int c = 0;
+#pragma unroll
+    for (int r = 0; r < WO_PER_THREAD; r++) {
+        const long i = base + r * WO_THREADS + threadIdx.x;
+        c += __syncthreads_count(i < n && type[i] == SPH_TYPE_FLUID);
+    }
+    if (threadIdx.x == 0) tiles[blockIdx.x] = (unsigned)c;
+}
+
+__global__ void __launch_bounds__(1024)
+k_fluid_scan(int tiles, unsigned* __restrict__ cnt, const unsigned* gate) {
+    __shared__ unsigned s_w[32];
+    if (gated_off(gate)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned carry = 0;
+    for (int base = 0; base < tiles; base += 1024) {
+        const int i = base + tid;
+        const unsigned v = i < tiles ? cnt[i] : 0u;
+        unsigned incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_w[warp] = incl;
+        __syncthreads();
+        unsigned before = 0, all = 0;
+        for (int w = 0; w < 32; w++) {
+            if (w < warp) before += s_w[w];
+            all += s_w[w];
+        }
+        if (i < tiles) cnt[i] = carry + before + incl - v;
+        carry += all;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(WO_THREADS)
+k_fluid_rank(int n, const int* __restrict__ type, const unsigned* __restrict__ tiles,
+             int* __restrict__ rank, const unsigned* gate) {
+    __shared__ int s_w[WO_PER_THREAD][WO_THREADS / 32];
+    if (gated_off(gate)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long base = (long)blockIdx.x * WO_TILE;
+    unsigned mine[WO_PER_THREAD];
+#pragma unroll
+    for (int r = 0; r < WO_PER_THREAD; r++) {
+        const long i = base + r * WO_THREADS + tid;
+        mine[r] = __ballot_sync(0xffffffffu, i < n && type[i] == SPH_TYPE_FLUID);
+        if (lane == 0) s_w[r][warp] = __popc(mine[r]);
+    }
+    __syncthreads();
+    int run = (int)tiles[blockIdx.x];
+#pragma unroll
+    for (int r = 0; r < WO_PER_THREAD; r++) {
+        int before = run;
+        for (int w = 0; w < WO_THREADS / 32; w++) {
+            if (w < warp) before += s_w[r][w];
+            run += s_w[r][w];
+        }
+        const long i = base + r * WO_THREADS + tid;
+        if (i <= n) rank[i] = before + __popc(mine[r] & lanemask_lt());
+    }
+}
+
+// order[position of slot i] = i.  The fluid slots come first, then the others, each in slot order
+// or, with `rows`, with the rows y = 2m and 2m + 1 of a layer merged by cell x (a particle of the
+// even row before one of the odd row): consecutive positions then hold particles one above the
+// other.  The merged position is the rank in the own row plus the partner row's particles before
+// it, both from the dense cell starts.
+__global__ void k_work_order(int n, int gx, int gy, unsigned num_cells, int rows,
+                             const int* __restrict__ type, const int* __restrict__ rank,
+                             const unsigned* __restrict__ keys, const int* __restrict__ cs,
+                             int* __restrict__ order, const unsigned* gate) {
+    if (gated_off(gate)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const bool fluid = type[i] == SPH_TYPE_FLUID;
+    const int nf = rank[n];
+    // slots of i's kind before slot j
+    auto before = [&](int j) {
+        const int f = __ldg(rank + j);
+        return fluid ? f : j - f;
+    };
+    int pos = before(i);
+    const unsigned key = keys[i];
+    if (rows && key < num_cells) {
+        int cx, cy, cz;
+        cell_of_key(gx, gy, key, cx, cy, cz);
+        const int odd = cy & 1;
+        if (odd || cy + 1 < gy) {
+            auto start = [&](int c) { return before(min(max(__ldg(cs + c), 0), n)); };
+            const int own = (int)key - cx, other = odd ? own - gx : own + gx;
+            // the partner row's particles before i, against those the slot order has before it
+            const int ahead = start(other + cx + odd) - start(other);
+            pos += odd ? ahead - (start(own) - start(other)) : ahead;
+        }
+    }
+    if (!fluid) pos += nf;
+    if ((unsigned)pos < (unsigned)n) order[pos] = i;
+}
+
 // Instance of particle i when instance b owns [off[b], off[b+1]) (upper bound search).
 __device__ __forceinline__ int instance_of(const int* __restrict__ off, int n_inst, int i) {
     if (!off || n_inst <= 1) return 0;
@@ -759,6 +873,20 @@ cudaError_t build_cell_starts(const unsigned* sorted_keys, int n, int num_cells,
                                                        fluid_cells);
     k_cell_fill<<<blocks_for((long)num_cells + 1, FILL_CHUNK), FILL_THREADS, 0, s>>>(
         cs, num_cells, sorted_keys, n, gate);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int* type,
+                              const unsigned* keys, const int* cs, int* rank, unsigned* tiles,
+                              int* order, cudaStream_t s, const unsigned* gate) {
+    if (n <= 0) return cudaSuccess;
+    const int nt = blocks_for((long)n + 1, WO_TILE);
+    k_fluid_count<<<nt, WO_THREADS, 0, s>>>(n, type, tiles, gate);
+    k_fluid_scan<<<1, 1024, 0, s>>>(nt, tiles, gate);
+    k_fluid_rank<<<nt, WO_THREADS, 0, s>>>(n, type, tiles, rank, gate);
+    k_work_order<<<blocks_for(n, 256), 256, 0, s>>>(n, grid.grid_dim[0], grid.grid_dim[1],
+                                                    (unsigned)grid.num_cells, rows, type, rank,
+                                                    keys, cs, order, gate);
     return cudaGetLastError();
 }
 

@@ -11,6 +11,13 @@ namespace {
 
 constexpr double kPi = 3.141592654;  // the reference's PI (src/header/sph.cuh:4)
 
+// An FP32 value in both halves of a two-lane operand.
+unsigned long long twice(float v) {
+    unsigned u;
+    std::memcpy(&u, &v, sizeof(u));
+    return (unsigned long long)u << 32 | u;
+}
+
 void fill_grid(sph_params* P, double pad, const float dmin[3], const float dmax[3]) {
     for (int c = 0; c < 3; c++) {
         P->grid_min[c] = (float)((double)dmin[c] - pad);
@@ -81,6 +88,15 @@ KParams make_kparams(const sph_params& p, int n) {
     k.park_z = p.escape_park[2];
     k.park_inactive = p.park_inactive;
     k.inst_boxes = 0;
+    k.inv_h2 = twice(k.inv_h);
+    k.m_half_inv_h2 = twice(-0.5f * k.inv_h);
+    k.one2 = twice(1.f);
+    k.m_half2 = twice(-0.5f);
+    k.c_fr2 = twice(k.c_fr);
+    k.c_fr_mass2 = twice(k.c_fr_mass);
+    k.eta2_2 = twice(k.eta2);
+    k.delta_h_cs2 = twice(k.delta_h_cs);
+    k.visc2 = twice(k.visc);
     return k;
 }
 

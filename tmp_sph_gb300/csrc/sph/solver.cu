@@ -52,7 +52,7 @@ void free_set(ParticleSetT<T>& s) {
 template <class T>
 cudaError_t alloc_set(ParticleSetT<T>& s, int cap, bool mixed) {
     cudaError_t e;
-    if ((e = dalloc(&s.rec, 2 * (size_t)cap)) != cudaSuccess) return e;
+    if ((e = dalloc(&s.rec, 2 * ((size_t)cap + 1))) != cudaSuccess) return e;
     if ((e = dalloc(&s.xyz, cap)) != cudaSuccess) return e;
     if ((e = dalloc(&s.type, cap)) != cudaSuccess) return e;
     if ((e = dalloc(&s.id, cap)) != cudaSuccess) return e;
@@ -75,7 +75,7 @@ void free_p1(Pass1OutT<T>& p) {
 
 template <class T>
 cudaError_t alloc_p1(Pass1OutT<T>& p, int cap) {
-    cudaError_t e = dalloc(&p.nrec, 2 * (size_t)cap);
+    cudaError_t e = dalloc(&p.nrec, 2 * ((size_t)cap + 1));
     if (e == cudaSuccess) e = dalloc(&p.self, cap);
     return e;
 }
@@ -216,6 +216,7 @@ bool per_instance(const sph_ctx* c) {
 // The neighbour list to use this half step, or NULL to walk the cells in every pass.
 const NbrList* list_for(sph_ctx* c) {
     c->nl.fluid_cells = c->fluid_cells;
+    c->nl.order = c->perm;
     const bool pi = per_instance(c);
     c->nl.iw = pi ? c->iw : nullptr;
     c->nl.inst = pi ? (c->prec == SPH_PREC_FP64 ? c->yd.inst : c->y.inst) : nullptr;
@@ -287,11 +288,8 @@ static int pass1_lanes(const sph_ctx* c) {
 // (SPH_PREC_MIXED_ABS), which share the FP32 defaults below.
 static bool fp32_pairs(int prec) { return prec == SPH_PREC_FP32 || prec == SPH_PREC_MIXED_ABS; }
 
-// Threads per block of the neighbour kernels: the option, or by default 256 in FP32 (their
-// static shared memory is sized for 256 threads, so 128-thread blocks pack twice as much per
-// SM and leave L1 less room: 4.96M dam break 3.26 against 3.32 ms per step, 7.50 against 7.60
-// rebuilding every half step) and 128 in the other precisions (mixed precision's 56-register
-// pass 2 keeps 36 warps per SM in 128-thread blocks, 32 in 256: 3.64 against 3.75 ms).
+// Threads per block of the neighbour kernels: the option, or by default 256 in FP32 (their static
+// shared memory is sized for 256 threads) and 128 in the other precisions.
 static int block_threads(const sph_ctx* c) {
     if (c->opt_threads > 0) return c->opt_threads;
     return fp32_pairs(c->prec) ? 256 : 128;
@@ -571,9 +569,15 @@ cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, cudaStre
                                y.type, c->fluid_cells)) !=
         cudaSuccess)
         return e;
+    // the permutation just applied, the sort's scratch and the pass-1 records hold nothing now
+    if (nl && (e = launch_work_order(c->n, c->Pi, 0, y.type, c->keys_sorted,
+                                     c->cell_start, reinterpret_cast<int*>(State<P>::p1(c).self),
+                                     static_cast<unsigned*>(c->sort_scratch), c->perm, s,
+                                     gate)) != cudaSuccess)
+        return e;
     if (ev) cudaEventRecord(ev[PH_NBR], s);
-    if (nl && (e = launch_nbr_build<P>(k, y, c->keys_sorted, c->cell_start, *nl, 0, c->err, s,
-                                       gate)) != cudaSuccess)
+    if (nl && (e = launch_nbr_build<P>(k, y, c->keys_sorted, c->cell_start, *nl,
+                                       State<P>::p1(c).nrec, 0, c->err, s, gate)) != cudaSuccess)
         return e;
     return cudaSuccess;
 }
@@ -699,7 +703,7 @@ cudaError_t alloc_list(sph_ctx* c) {
     if (c->nl.idx && c->nl.cap == cap) return cudaSuccess;
     free_list(c->nl);
     // warp-interleaved blocks of cap x 32 slots: whole warps, the last one padded
-    const size_t rows = ((size_t)(c->capacity > 0 ? c->capacity : 1) + 31) & ~(size_t)31;
+    const size_t rows = ((size_t)(c->capacity > 0 ? c->capacity : 1) + 63) & ~(size_t)63;
     cudaError_t e = dalloc(&c->nl.idx, (size_t)cap * rows);
     if (e == cudaSuccess) e = dalloc(&c->nl.count, c->capacity);
     if (e == cudaSuccess) e = dalloc(&c->nl.xb, c->capacity);
@@ -1413,9 +1417,10 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
     NbrList dl = c->nl;
     dl.cut2 = nullptr;
     dl.fluid_cells = nullptr;
+    dl.order = nullptr;
     const NbrList* nl = list_for(c) ? &dl : nullptr;
     if (nl && launch_nbr_build<PrecF32>(k, c->x, c->keys_sorted, c->cell_start, *nl,
-                                        c->opt_wall_rates, c->err, s) != cudaSuccess)
+                                        c->p1.nrec, c->opt_wall_rates, c->err, s) != cudaSuccess)
         return SPH_ERR_CUDA;
     if (launch_pass1<PrecF32>(k, c->x, c->keys_sorted, c->cell_start, nl, c->p1, rhop_sum,
                               w_sum, s) != cudaSuccess)
