@@ -263,10 +263,14 @@ typedef struct sph_ctx sph_ctx;
 #define SPH_OPT_PRECISION     8  /* SPH_PREC_* below; set before sph_upload (the state is
                                     reallocated; the uploaded state is dropped) */
 #define SPH_OPT_BLOCK_THREADS 9  /* threads per block of the neighbour kernels: 32..256, a
-                                    multiple of 32; 0 (default): 256 in FP32, 128 in the
+                                    multiple of 32; 0 (default): 64 where a thread takes two
+                                    particles (below), else 256 in FP32 and 128 in the
                                     other precisions */
 #define SPH_OPT_PARTICLES_PER_THREAD 10  /* particles each thread of the neighbour kernels
-                                    handles, grid-stride (1..64, default 1) */
+                                    handles, grid-stride (1..64, default 1).  At the default,
+                                    FP32 and SPH_PREC_MIXED_ABS runs of 400,000 particles and more
+                                    with a neighbour list, one pass-1 lane and one rebuild decision
+                                    share each list and thread between two particles (same bits) */
 /* 11 is not used (it selected a two-particles-per-thread mode, measured slower and removed) */
 #define SPH_OPT_ADAPTIVE_SKIN 13  /* 1 (default): each list rebuild picks the skin of the next
                              lists, between 0.02 and SPH_OPT_SKIN_PERMILLE, from how long the

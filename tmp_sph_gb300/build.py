@@ -27,6 +27,7 @@ SOURCES = [
     "lib/sort_noalloc.cu",
     "equation/ns.cu",
     "equation/ns_groups.cu",
+    "equation/ns_twin.cu",
     "sph/integrator.cu",
     "sph/solver.cu",
     "sph/params.cpp",

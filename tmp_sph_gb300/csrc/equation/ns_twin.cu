@@ -1,0 +1,402 @@
+// ns_twin.cu — the neighbour list and both passes with two particles per thread, for the FP32 pair
+// arithmetic (FP32, and mixed precision on FP32 positions).
+//
+// Same pairs, same arithmetic and same order of every particle's sums as ns.cu (bit for bit);
+// another assignment of work to threads.  Thread u takes work positions 2u and 2u + 1 over one
+// list: the union of their neighbours in cell-walk order, about 1.3 times as long as either's.
+// Every record gathered serves both (two-lane instructions, one lane per particle, each sum under
+// the predicate of its own distance), so a particle costs 0.65 gathers per neighbour instead of
+// one: the passes with one particle per thread are bound by the L1 data stage and the latency of
+// those gathers.
+//
+// The two particles lie one above the other (the same x in rows y = 2m and 2m + 1; k_work_order
+// merges the rows): the lanes of a warp then still gather neighbouring records, 9.3 L1 wavefronts
+// a request.  Two neighbours of one row per thread have the same union but put the lanes two
+// records apart: 17 wavefronts, and pass 1 at 467 instead of 361 us (4.96M particles).
+//
+// Measured, pass 1 / pass 2 against one particle per thread with one gather in flight: 4.96M
+// particles 520 / 609 -> 361 / 582 us, a disordered surge of 6.70M 1020 / 1078 -> 750 / 927 us.
+// What is left is latency: pass 2 issues in 60-70% of cycles with 18 warps per SM (104 registers),
+// L1 data stage 45% (pass 1 70%).  Slower: 80 registers (630 us, the gathers of a chunk no longer
+// issued together), records of the next half chunk loaded during the current one (640-690 us),
+// lists prefetched into L2 ahead of their use (level).
+#include <cuda_runtime.h>
+
+#include "ns_pair.cuh"
+#include "sph_internal.h"
+
+namespace sph {
+
+namespace {
+
+// The two particles of thread u: slots a and b (b = a when u has one particle only).
+struct Twin {
+    int a, b;
+    bool two;
+};
+__device__ __forceinline__ Twin twin_of(const NbrList& nl, int u, int n) {
+    Twin w;
+    w.a = work_slot(nl, 2 * u);
+    w.two = 2 * u + 1 < n;
+    w.b = w.two ? work_slot(nl, 2 * u + 1) : w.a;
+    return w;
+}
+// Column of thread u's list: as nbr_col, with the slots of its two particles.
+__device__ __forceinline__ size_t twin_col(const NbrList& nl, int u) {
+    return (size_t)(u >> 5) * ((size_t)nl.cap << 6) + ((size_t)(u & 31) << 2);
+}
+constexpr int TWIN_WALKS = -1;  // count of a thread one of whose particles overflowed its list
+
+// ---------------------------------------------------------------- list build
+template <class KP>
+__device__ __forceinline__ bool near_fluid(const KP& k, const unsigned char* __restrict__ fluid,
+                                           int cx, int cy, int cz) {
+    const int r = k.reach;
+    bool any = false;
+    for (int z = max(cz - r, 0); z <= min(cz + r, k.gz - 1); z++)
+        for (int y = max(cy - r, 0); y <= min(cy + r, k.gy - 1); y++) {
+            const int row = (z * k.gy + y) * k.gx;
+            for (int x = max(cx - r, 0); x <= min(cx + r, k.gx - 1); x++)
+                any = any || __ldg(fluid + row + x) != 0;
+        }
+    return any;
+}
+
+// One particle's side of the build: its cell and the part of a strip its cutoff sphere reaches.
+struct TwinWalk {
+    int cx, cy, cz;
+    bool on;  // takes part in the neighbour search
+    StripWindow win;
+    template <class KP>
+    __device__ __forceinline__ bool strip(const KP& k, int y, int z, int& xl, int& xh) const {
+        const int r = k.reach;
+        if (!on || abs(z - cz) > r || abs(y - cy) > r) return false;
+        xl = max(cx - r, 0);
+        xh = min(cx + r, k.gx - 1);
+        return win(y, z, xl, xh);
+    }
+};
+
+template <class P>
+__device__ __forceinline__ TwinWalk twin_walk(const KParamsT<float>& k, const float4& p,
+                                              unsigned key, float cut2) {
+    TwinWalk w;
+    w.on = !inactive_key(k, key);
+    cell_of_key(k.gx, k.gy, w.on ? key : 0u, w.cx, w.cy, w.cz);
+    w.win = strip_window<P>(k, p, w.cx, w.cy, w.cz, cut2);
+    return w;
+}
+
+constexpr int TWIN_BUILD_THREADS = 128;
+
+template <class P>
+__global__ void __launch_bounds__(TWIN_BUILD_THREADS)
+k_nbr_build_twin(KParamsT<float> k, const float4* __restrict__ X,
+                 const unsigned* __restrict__ keys, const int* __restrict__ cs, NbrList nl,
+                 float4* rec, float4* nrec, unsigned* err, const unsigned* gate) {
+    __shared__ int4 s_stage[TWIN_BUILD_THREADS];
+    if (gated_off(gate)) return;
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u == 0) {
+        pad_record<float>(rec, k.n);
+        pad_record<float>(nrec, k.n);
+    }
+    if (2 * u >= k.n) return;
+    const float cut2 = nl.cut2 ? __ldg(nl.cut2) : k.kh2_list;
+    const Twin tw = twin_of(nl, u, k.n);
+    const int a = tw.a, b = tw.b;
+    const float4 pa = X[a], pb = X[b];
+    if (nl.xb) {
+        nl.xb[a] = pa;
+        nl.xb[b] = pb;
+    }
+    const bool alla = fluid_rec(pa.w), allb = fluid_rec(pb.w);
+    const TwinWalk wa = twin_walk<P>(k, pa, keys[a], cut2), wb = twin_walk<P>(k, pb, keys[b], cut2);
+    if (!alla && !allb && nl.fluid_cells &&
+        !(wa.on && near_fluid(k, nl.fluid_cells, wa.cx, wa.cy, wa.cz)) &&
+        !(wb.on && near_fluid(k, nl.fluid_cells, wb.cx, wb.cy, wb.cz))) {
+        nl.count[u] = 0;
+        return;
+    }
+    SlotWriter<false> w(nl.idx + twin_col(nl, u), 2 * nl.cap, s_stage);
+    int na = 0, nb = 0;
+    auto run = [&](int row, int x0, int x1) {
+        const int j0 = max(__ldg(cs + row + x0), 0);
+        const int j1 = min(__ldg(cs + row + x1 + 1), k.n);  // bounds guard only
+#pragma unroll 4
+        for (int j = j0; j < j1; j++) {
+            const float4 pj = ld_pos(X, (size_t)j);
+            float ax, ay, az, bx, by, bz;
+            rel_pos<P>(k, pa, pj, 0u, ax, ay, az);
+            rel_pos<P>(k, pb, pj, 0u, bx, by, bz);
+            const bool fj = fluid_rec(pj.w);
+            const bool ia = dist2(ax, ay, az) < cut2 && j != a && (alla || fj);
+            const bool ib = dist2(bx, by, bz) < cut2 && j != b && (allb || fj);
+            na += ia;
+            nb += ib;
+            if (ia || ib) w.put(j);
+        }
+    };
+    // the strips of either particle in (z, y) order, each particle's cells of a strip in x order
+    const int r = k.reach;
+    const int za = wa.on ? wa.cz : wb.cz, zb = wb.on ? wb.cz : wa.cz;
+    const int z1 = min(max(za, zb) + r, k.gz - 1);
+    if (wa.on || wb.on)
+#pragma unroll 1
+        for (int z = max(min(za, zb) - r, 0); z <= z1; z++) {
+            const bool ina = wa.on && abs(z - wa.cz) <= r, inb = wb.on && abs(z - wb.cz) <= r;
+            if (!ina && !inb) {  // between two particles far apart
+                z = max(za, zb) - r - 1;
+                continue;
+            }
+            const int ya = ina ? wa.cy : wb.cy, yb = inb ? wb.cy : wa.cy;
+            const int y1 = min(max(ya, yb) + r, k.gy - 1);
+#pragma unroll 1
+            for (int y = max(min(ya, yb) - r, 0); y <= y1; y++) {
+                if (abs(y - ya) > r && abs(y - yb) > r) {
+                    y = max(ya, yb) - r - 1;
+                    continue;
+                }
+                int la, ha, lb, hb;
+                const bool sa = wa.strip(k, y, z, la, ha), sb = wb.strip(k, y, z, lb, hb);
+                const int row = (z * k.gy + y) * k.gx;
+                if (sa && sb) {
+                    const int l = min(la, lb), h = max(ha, hb);
+                    const int cut = min(ha, hb), next = max(la, lb);
+                    if (next <= cut + 1) {
+                        run(row, l, h);
+                    } else {  // two separate runs of one strip
+                        run(row, l, cut);
+                        run(row, next, h);
+                    }
+                } else if (sa) {
+                    run(row, la, ha);
+                } else if (sb) {
+                    run(row, lb, hb);
+                }
+            }
+        }
+    w.flush(pad_slot<P>(k.n));
+    const bool over = na > nl.cap || nb > nl.cap;
+    nl.count[u] = over ? TWIN_WALKS : w.cnt;
+    raise_flags(err, over ? SPH_FLAG_NEIGHBOR_OVERFLOW : 0u);
+}
+
+// ---------------------------------------------------------------- passes
+// The records of thread u's list, four gathers issued together: one(a, v) for each in order.
+template <class F>
+__device__ __forceinline__ void visit_twin(const NbrList& nl, const float4* __restrict__ R, int u,
+                                           int cnt, F&& one) {
+    for_each_chunk<false>(nl.idx + twin_col(nl, u), cnt, 0, 1, [&](const int4& q) {
+        const int e[4] = {q.x, q.y, q.z, q.w};
+        float4 a[4], v[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) ld_rec(R, e[c], a[c], v[c]);
+#pragma unroll
+        for (int c = 0; c < 4; c++) one(a[c], v[c]);
+    });
+}
+
+// Pass-1 sums of two fluid particles and one neighbour (Pass1Acc::pair of each).
+template <class P>
+__device__ __forceinline__ void pass1_twin(const KParamsT<float>& k, Pass1Acc<P>& A,
+                                           Pass1Acc<P>& B, const float4& aj, const float4& vj) {
+    float ax, ay, az, bx, by, bz;
+    rel_pos<P>(k, A.pi, aj, 0u, ax, ay, az);
+    rel_pos<P>(k, B.pi, aj, 0u, bx, by, bz);
+    const float r2a = dist2(ax, ay, az), r2b = dist2(bx, by, bz);
+    const F2 rr = pack2(pair_sqrt(r2a), pair_sqrt(r2b));
+    const F2 t = fma2_rn(F2{k.m_half2}, mul2_rn(rr, F2{k.inv_h2}), F2{k.one2});
+    const F2 fr = mul2_rn(mul2_rn(F2{k.c_fr2}, mul2_rn(t, t)), t);
+    const F2 vdotr = pack2(dot_rn(A.vi, vj, ax, ay, az), dot_rn(B.vi, vj, bx, by, bz));
+    float ua, ub;
+    unpack2(mul2_rn(fr, vdotr), ua, ub);
+    const float m = mul_rn(k.mass, pair_rcp(vj.w));
+    add_if(r2a, k.kh2, vj.w, -ua, m, A.dofv.s);
+    add_if(r2b, k.kh2, vj.w, -ub, m, B.dofv.s);
+}
+
+// Pass-2 sums of two fluid particles and one neighbour (Pass2Acc::pair of each).
+template <class P, int MODE>
+__device__ __forceinline__ void pass2_twin(const KParamsT<float>& k, Pass2Acc<P, MODE>& A,
+                                           Pass2Acc<P, MODE>& B, const float4& aj,
+                                           const float4& vj) {
+    float ax, ay, az, sa, bx, by, bz, sb;
+    rel_pos_s<P>(k, A.pi, -A.presi, aj, 0u, ax, ay, az, sa);
+    rel_pos_s<P>(k, B.pi, -B.presi, aj, 0u, bx, by, bz, sb);
+    const float r2a = dist2(ax, ay, az), r2b = dist2(bx, by, bz);
+    const F2 r2 = pack2(r2a, r2b);
+    const float rhoj = dabs(vj.w);
+    const F2 rr = pack2(pair_sqrt(r2a), pair_sqrt(r2b));
+    const F2 t = fma2_rn(F2{k.m_half_inv_h2}, rr, F2{k.one2});
+    float wa, wb, ea, eb;
+    unpack2(mul2_rn(mul2_rn(F2{k.c_fr_mass2}, mul2_rn(t, t)), t), wa, wb);
+    const float rj = pair_rcp(rhoj);
+    wa = mul_rn(wa, rj);
+    wb = mul_rn(wb, rj);
+    const F2 vdotr = pack2(dot_rn(A.vi, vj, ax, ay, az), dot_rn(B.vi, vj, bx, by, bz));
+    unpack2(add2_rn(r2, F2{k.eta2_2}), ea, eb);
+    const F2 inv = pack2(pair_rcp(ea), pair_rcp(eb));
+    const F2 dr = pack2(sub_rn(A.rhoi, rhoj), sub_rn(B.rhoi, rhoj));
+    const F2 diff = mul2_rn(mul2_rn(mul2_rn(dr, F2{k.delta_h_cs2}), r2), inv);
+    unpack2(fma2_rn(pack2(A.rhoi, B.rhoi), vdotr, diff), ea, eb);
+    float va, vb;
+    unpack2(fma2_rn(mul2_rn(F2{k.visc2}, vdotr), inv, pack2(A.damp_i, B.damp_i)), va, vb);
+    const bool fj = fluid_rec(vj.w);
+    const float ca = mul_rn(wa, fj ? add_rn(sa, va) : sa), cb = mul_rn(wb, fj ? add_rn(sb, vb) : sb);
+    add_if(r2a, k.kh2, wa, ea, ca, ax, ay, az, A.sd.s, A.sx.s, A.sy.s, A.sz.s);
+    add_if(r2b, k.kh2, wb, eb, cb, bx, by, bz, B.sd.s, B.sx.s, B.sy.s, B.sz.s);
+}
+
+template <class P>
+__global__ void __maxnreg__(80)
+k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ keys,
+             const int* __restrict__ cs, NbrList nl, Pass1Out out) {
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (2 * u >= k.n) return;
+    const Twin tw = twin_of(nl, u, k.n);
+    Pass1Acc<P> A, B;
+    A.load(in.rec, tw.a);
+    B.load(in.rec, tw.b);
+    const int cnt = __ldg(nl.count + u);
+    if (cnt >= 0) {
+        if (A.fi || B.fi) {
+            visit_twin(nl, in.rec, u, cnt, [&](const float4& aj, const float4& vj) {
+                pass1_twin<P>(k, A, B, aj, vj);
+            });
+            if (!A.fi) A.dofv.s = 0.f;
+            if (!B.fi) B.dofv.s = 0.f;
+        }
+        if (!A.fi || !B.fi) {
+            visit_twin(nl, in.rec, u, cnt, [&](const float4& aj, const float4& vj) {
+                float dx, dy, dz;
+                rel_pos<P>(k, A.pi, aj, 0u, dx, dy, dz);
+                float r2 = dist2(dx, dy, dz);
+                if (!A.fi && r2 < k.kh2) A.pair(k, aj, vj, dx, dy, dz, r2);
+                rel_pos<P>(k, B.pi, aj, 0u, dx, dy, dz);
+                r2 = dist2(dx, dy, dz);
+                if (!B.fi && r2 < k.kh2) B.pair(k, aj, vj, dx, dy, dz, r2);
+            });
+        }
+    } else {
+#pragma unroll 1
+        for (int m = 0; m < 2; m++) {
+            Pass1Acc<P> C = m ? B : A;
+            walk_pairs<P, 1>(k, cs, keys, in.xyz, m ? tw.b : tw.a, C.pi, k.kh2,
+                             [&](int j, unsigned, const float4&, float dx, float dy, float dz,
+                                 float r2) {
+                float4 aj, vj;
+                ld_rec(in.rec, j, aj, vj);
+                C.pair(k, aj, vj, dx, dy, dz, r2);
+            });
+            if (m) B = C;
+            else A = C;
+        }
+    }
+    A.template finish<false>(k, out, nullptr, nullptr, tw.a);
+    if (tw.two) B.template finish<false>(k, out, nullptr, nullptr, tw.b);
+}
+
+template <class P, int MODE>
+__global__ void __maxnreg__(104)
+k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ keys,
+             const int* __restrict__ cs, NbrList nl, Pass1Out p1, ParticleSet out,
+             unsigned* __restrict__ out_hash, unsigned* err, unsigned* disp) {
+    DispBox box;
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (2 * u < k.n) {
+        const Twin tw = twin_of(nl, u, k.n);
+        Pass2Acc<P, MODE> A, B;
+        A.load(k, p1, tw.a, 0);
+        B.load(k, p1, tw.b, 0);
+        if (A.active || B.active) {
+            const int cnt = __ldg(nl.count + u);
+            if (cnt >= 0) {
+                visit_twin(nl, p1.nrec, u, cnt, [&](const float4& aj, const float4& vj) {
+                    pass2_twin<P, MODE>(k, A, B, aj, vj);
+                });
+            } else {
+#pragma unroll 1
+                for (int m = 0; m < 2; m++) {
+                    Pass2Acc<P, MODE> C = m ? B : A;
+                    if (C.active)
+                        walk_pairs<P, 2>(k, cs, keys, p1.nrec, m ? tw.b : tw.a, C.pi, k.kh2,
+                                         [&](int j, unsigned, const float4&, float dx, float dy,
+                                             float dz, float r2) {
+                            float4 aj, vj;
+                            ld_rec(p1.nrec, j, aj, vj);
+                            C.pair(k, p1, j, aj, vj, dx, dy, dz, r2);
+                        });
+                    if (m) B = C;
+                    else A = C;
+                }
+            }
+        }
+#pragma unroll 1
+        for (int m = 0; m < (tw.two ? 2 : 1); m++) {
+            const Pass2Acc<P, MODE> C = m ? B : A;
+            pass2_finish<P, MODE>(k, m ? tw.b : tw.a, C, in, keys, nl, nullptr, nullptr, 0, out,
+                                  out_hash, err, box, disp);
+        }
+    }
+    if (disp == nullptr) return;
+    // the block's displacement box; blockDim is a multiple of 32, every thread gets here
+    __shared__ unsigned s_box[6 * (NS_MAX_THREADS / 32)];
+    reduce_disp_box(box, disp, s_box);
+}
+
+inline int twin_blocks(int n, int threads) { return (n + 2 * threads - 1) / (2 * threads); }
+
+}  // namespace
+
+template <class P>
+cudaError_t launch_nbr_build_twin(const KParams& k, const ParticleSet& in, const unsigned* keys,
+                                  const int* cs, const NbrList& nl, float4* nrec, unsigned* err,
+                                  cudaStream_t s, const unsigned* gate) {
+    if (k.n <= 0) return cudaSuccess;
+    k_nbr_build_twin<P><<<twin_blocks(k.n, TWIN_BUILD_THREADS), TWIN_BUILD_THREADS, 0, s>>>(
+        k, in.xyz, keys, cs, nl, in.rec, nrec, err, gate);
+    return cudaGetLastError();
+}
+
+template <class P>
+cudaError_t launch_pass1_twin(const KParams& k, const ParticleSet& in, const unsigned* keys,
+                              const int* cs, const NbrList& nl, const Pass1Out& out,
+                              cudaStream_t s) {
+    if (k.n <= 0) return cudaSuccess;
+    k_pass1_twin<P><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(k, in, keys, cs, nl, out);
+    return cudaGetLastError();
+}
+
+template <class P>
+cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet& in,
+                              const unsigned* keys, const int* cs, const NbrList& nl,
+                              const Pass1Out& p1, ParticleSet out, unsigned* out_hash,
+                              unsigned* err, unsigned* disp, cudaStream_t s) {
+    if (k.n <= 0) return cudaSuccess;
+    if (half == HALF_PREDICT)
+        k_pass2_twin<P, MODE_PRED><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(
+            k, in, keys, cs, nl, p1, out, out_hash, err, disp);
+    else
+        k_pass2_twin<P, MODE_CORR><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(
+            k, in, keys, cs, nl, p1, out, out_hash, err, disp);
+    return cudaGetLastError();
+}
+
+#define SPH_NS_TWIN_INSTANTIATE(P)                                                             \
+    template cudaError_t launch_nbr_build_twin<P>(const KParams&, const ParticleSet&,          \
+                                                  const unsigned*, const int*, const NbrList&, \
+                                                  float4*, unsigned*, cudaStream_t,            \
+                                                  const unsigned*);                            \
+    template cudaError_t launch_pass1_twin<P>(const KParams&, const ParticleSet&,              \
+                                              const unsigned*, const int*, const NbrList&,     \
+                                              const Pass1Out&, cudaStream_t);                  \
+    template cudaError_t launch_pass2_twin<P>(const KParams&, HalfStep, const ParticleSet&,    \
+                                              const unsigned*, const int*, const NbrList&,     \
+                                              const Pass1Out&, ParticleSet, unsigned*,         \
+                                              unsigned*, unsigned*, cudaStream_t);
+SPH_NS_TWIN_INSTANTIATE(PrecF32)
+SPH_NS_TWIN_INSTANTIATE(PrecMixA)
+#undef SPH_NS_TWIN_INSTANTIATE
+
+}  // namespace sph

@@ -214,6 +214,22 @@ cudaError_t launch_pass2_step(const KParamsT<typename P::T>& k, HalfStep half,
                               ParticleSetT<typename P::T> out, unsigned* out_hash, unsigned* err,
                               unsigned* disp, cudaStream_t s);
 
+// Two particles per thread (equation/ns_twin.cu): the list build and both passes for the FP32
+// pair arithmetic without cell codes, over lists shared by work positions 2u and 2u + 1.
+template <class P>
+cudaError_t launch_nbr_build_twin(const KParams& k, const ParticleSet& in, const unsigned* keys,
+                                  const int* cs, const NbrList& nl, float4* nrec, unsigned* err,
+                                  cudaStream_t s, const unsigned* gate);
+template <class P>
+cudaError_t launch_pass1_twin(const KParams& k, const ParticleSet& in, const unsigned* keys,
+                              const int* cs, const NbrList& nl, const Pass1Out& out,
+                              cudaStream_t s);
+template <class P>
+cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet& in,
+                              const unsigned* keys, const int* cs, const NbrList& nl,
+                              const Pass1Out& p1, ParticleSet out, unsigned* out_hash,
+                              unsigned* err, unsigned* disp, cudaStream_t s);
+
 // Resident-state glue (lib/mesh.cu), one instantiation per precision policy P.
 // perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
 // cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).

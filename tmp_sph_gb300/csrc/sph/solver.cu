@@ -288,10 +288,27 @@ static int pass1_lanes(const sph_ctx* c) {
 // (SPH_PREC_MIXED_ABS), which share the FP32 defaults below.
 static bool fp32_pairs(int prec) { return prec == SPH_PREC_FP32 || prec == SPH_PREC_MIXED_ABS; }
 
-// Threads per block of the neighbour kernels: the option, or by default 256 in FP32 (their static
-// shared memory is sized for 256 threads) and 128 in the other precisions.
+// Whether the lists and passes take two particles per thread (equation/ns_twin.cu): the FP32 pair
+// arithmetic, one pass-1 lane, the default of one particle per thread, one rebuild decision for
+// all slots, and enough particles to fill the GPU with half the threads: at 380,000 particles the
+// two forms are level (5 steps 0.93 ms against 0.89 in a calm flow, 1.11 against 1.18 in a
+// disordered one), at 200,000 one particle per thread wins (0.70 against 0.57), at 766,000 two do
+// (1.60 against 1.75).  Both give the same bits.
+constexpr int TWIN_MIN_PARTICLES = 400000;
+static bool twin_lists(const sph_ctx* c) {
+    return fp32_pairs(c->prec) && c->opt_nbr_list && c->nl.idx && pass1_lanes(c) == 1 &&
+           c->opt_ppt == 1 && !per_instance(c) && c->n >= TWIN_MIN_PARTICLES;
+}
+template <class P>
+constexpr bool kTwin = P::kId == SPH_PREC_FP32 || P::kId == SPH_PREC_MIXED_ABS;
+
+// Threads per block of the neighbour kernels: the option, or by default 64 with two particles per
+// thread (104 registers a thread: nine blocks per SM; 128 threads: pass 2 596 against 582 us at
+// 4.96M particles), else 256 in FP32 (their static shared memory is sized for 256 threads) and 128
+// in the other precisions.
 static int block_threads(const sph_ctx* c) {
     if (c->opt_threads > 0) return c->opt_threads;
+    if (twin_lists(c)) return 64;
     return fp32_pairs(c->prec) ? 256 : 128;
 }
 
@@ -570,12 +587,17 @@ cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, cudaStre
         cudaSuccess)
         return e;
     // the permutation just applied, the sort's scratch and the pass-1 records hold nothing now
-    if (nl && (e = launch_work_order(c->n, c->Pi, 0, y.type, c->keys_sorted,
+    if (nl && (e = launch_work_order(c->n, c->Pi, twin_lists(c) ? 1 : 0, y.type, c->keys_sorted,
                                      c->cell_start, reinterpret_cast<int*>(State<P>::p1(c).self),
                                      static_cast<unsigned*>(c->sort_scratch), c->perm, s,
                                      gate)) != cudaSuccess)
         return e;
     if (ev) cudaEventRecord(ev[PH_NBR], s);
+    if constexpr (kTwin<P>) {
+        if (twin_lists(c))
+            return launch_nbr_build_twin<P>(k, y, c->keys_sorted, c->cell_start, *nl, c->p1.nrec,
+                                            c->err, s, gate);
+    }
     if (nl && (e = launch_nbr_build<P>(k, y, c->keys_sorted, c->cell_start, *nl,
                                        State<P>::p1(c).nrec, 0, c->err, s, gate)) != cudaSuccess)
         return e;
@@ -634,6 +656,18 @@ cudaError_t half_step(sph_ctx* c, HalfStep half, cudaStream_t s, cudaEvent_t* ev
     e = cc ? capture_conditional_rebuild<P>(c, k, s, *cc) : rebuild_lists<P>(c, k, s, ev);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[PH_PASS1], s);
+    if constexpr (kTwin<P>) {
+        if (twin_lists(c)) {
+            if ((e = launch_pass1_twin<P>(k, y, c->keys_sorted, c->cell_start, *nl, p1, s)) !=
+                cudaSuccess)
+                return e;
+            if (ev) cudaEventRecord(ev[PH_PASS2], s);
+            e = launch_pass2_twin<P>(k, half, y, c->keys_sorted, c->cell_start, *nl, p1, y,
+                                     c->hash_x, c->err, disp_words(c), s);
+            if (ev) cudaEventRecord(ev[PH_COUNT], s);
+            return e;
+        }
+    }
     if ((e = launch_pass1<P>(k, y, c->keys_sorted, c->cell_start, nl, p1, nullptr, nullptr,
                              s)) != cudaSuccess)
         return e;
@@ -861,9 +895,14 @@ extern "C" int sph_ctx_set_option(sph_ctx* c, int option, int value) {
             return SPH_OK;
         case SPH_OPT_PARTICLES_PER_THREAD:
             if (value < 1 || value > 64) return SPH_ERR_ARG;
+            if ((value > 1) == (c->opt_ppt > 1)) {
+                c->opt_ppt = value;
+                drop_graph(c);
+                return SPH_OK;
+            }
             c->opt_ppt = value;
             drop_graph(c);
-            return SPH_OK;
+            break;  // the lists may change form: rebuild
         case SPH_OPT_ADAPTIVE_SKIN:
             c->opt_adaptive_skin = value != 0;
             if (reset_skin_sync(c) != cudaSuccess) return SPH_ERR_CUDA;
