@@ -264,8 +264,8 @@ typedef struct sph_ctx sph_ctx;
                                     reallocated; the uploaded state is dropped) */
 #define SPH_OPT_BLOCK_THREADS 9  /* threads per block of the neighbour kernels: 32..256, a
                                     multiple of 32; 0 (default): 64 where a thread takes two
-                                    particles (below), else 256 in FP32 and 128 in the
-                                    other precisions */
+                                    particles (below), 32 in FP64, else 256 in FP32 below
+                                    60,000 particles and 128 */
 #define SPH_OPT_PARTICLES_PER_THREAD 10  /* particles each thread of the neighbour kernels
                                     handles, grid-stride (1..64, default 1).  At the default,
                                     FP32 and SPH_PREC_MIXED_ABS runs of 400,000 particles and more

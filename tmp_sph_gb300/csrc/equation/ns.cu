@@ -93,7 +93,7 @@ __device__ __forceinline__ void visit_fluid(const KParamsT<float>& k, const NbrL
 
 // Neighbours of slot i (work position t; r2 < kh2) with their records R[2j], R[2j+1]: from the list (pairs in the skin
 // beyond the support radius are skipped), or by walking the cells over X[XSTRIDE * j] when i
-// overflowed the list.  f(j, a, b, dx, dy, dz, r2); with FAST and kPairTwo the list goes through
+// overflowed the list.  f(j, a, b, dx, dy, dz, r2, vol); with FAST and kPairTwo the list goes through
 // acc.fluid_two instead (a fluid particle).
 template <class P, int LIST, int XSTRIDE, class Acc, class F>
 __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
@@ -101,8 +101,9 @@ __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
                                               const unsigned* __restrict__ keys,
                                               const NbrList& nl,
                                               const vec4_t<typename P::T>* __restrict__ X,
-                                              const vec4_t<typename P::T>* __restrict__ R, int t,
-                                              int i, Acc& acc, F&& f) {
+                                              const vec4_t<typename P::T>* __restrict__ R,
+                                              const typename P::T* __restrict__ vol, int t, int i,
+                                              Acc& acc, F&& f) {
     using T = typename P::T;
     using V = vec4_t<T>;
     if constexpr (LIST != LIST_NONE) {
@@ -121,7 +122,7 @@ __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
                 T dx, dy, dz;
                 rel_pos<P>(k, acc.pi, a, P::kCodes ? slot_code(e) : 0u, dx, dy, dz);
                 const T r2 = dist2(dx, dy, dz);
-                if (r2 < k.kh2) f(j, a, b, dx, dy, dz, r2);
+                if (inside(r2, k.kh2)) f(j, a, b, dx, dy, dz, r2, ld_vol(vol, j));
             };
             for_each_chunk<LIST == LIST_WIN>(nl.idx + nbr_col(nl, t), cnt, 0, 1,
                                              [&](const int4& q) {
@@ -137,7 +138,7 @@ __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
                            [&](int j, unsigned, const V&, T dx, T dy, T dz, T r2) {
         V a, b;
         ld_rec(R, j, a, b);
-        f(j, a, b, dx, dy, dz, r2);
+        f(j, a, b, dx, dy, dz, r2, ld_vol(vol, j));
     });
 }
 
@@ -269,9 +270,9 @@ __device__ __forceinline__ void pass1_one(const KParamsT<typename P::T>& k,
     const int i = work_slot(nl, t);
     Pass1Acc<P> acc;
     acc.load(in.rec, i);
-    visit_records<P, LIST, 1>(k, cs, keys, nl, in.xyz, in.rec, t, i, acc,
-                              [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
-        acc.pair(k, aj, vj, dx, dy, dz, r2);
+    visit_records<P, LIST, 1>(k, cs, keys, nl, in.xyz, in.rec, in.vol, t, i, acc,
+                              [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2, T vol) {
+        acc.pair(k, aj, vj, dx, dy, dz, r2, vol);
     });
     acc.template finish<WRITE_SUMS>(k, out, rhop_sum, w_sum, i);
 }
@@ -309,9 +310,10 @@ __device__ __forceinline__ void pass2_one(const KParamsT<typename P::T>& k, int 
     Pass2Acc<P, MODE> acc;
     acc.load(k, p1, i, wall_rates);
     if (acc.active)
-        visit_records<P, LIST, 2>(k, cs, keys, nl, p1.nrec, p1.nrec, t, i, acc,
-                                  [&](int j, const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
-            acc.pair(k, p1, j, aj, vj, dx, dy, dz, r2);
+        visit_records<P, LIST, 2>(k, cs, keys, nl, p1.nrec, p1.nrec, p1.vol, t, i, acc,
+                                  [&](int j, const V& aj, const V& vj, T dx, T dy, T dz, T r2,
+                                      T vol) {
+            acc.pair(k, p1, j, aj, vj, dx, dy, dz, r2, vol);
         });
     pass2_finish<P, MODE>(k, i, acc, in, keys, nl, rho_dt, vel_dt, wall_rates, out, out_hash,
                           err, box, disp);

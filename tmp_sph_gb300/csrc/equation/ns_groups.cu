@@ -70,14 +70,15 @@ __device__ __forceinline__ Sum<T, COMP> sum_of(T v) {
 // ---------------------------------------------------------------- neighbour visits
 // The group's share of particle i's neighbours (r2 < kh2) with their records: from the list,
 // lane s taking chunks s, s + G, ... of four entries; or, when i overflowed the list, by walking
-// the cells over X[XSTRIDE * j], G candidates per step.  f(j, a, b, dx, dy, dz, r2).
+// the cells over X[XSTRIDE * j], G candidates per step.  f(j, a, b, dx, dy, dz, r2, vol).
 template <class P, int G, int XSTRIDE, class F>
 __device__ __forceinline__ void visit_group(const KParamsT<typename P::T>& k,
                                             const int* __restrict__ cs,
                                             const unsigned* __restrict__ keys,
                                             const NbrList& nl,
                                             const vec4_t<typename P::T>* __restrict__ X,
-                                            const vec4_t<typename P::T>* __restrict__ R, int t, int i,
+                                            const vec4_t<typename P::T>* __restrict__ R,
+                                            const typename P::T* __restrict__ vol, int t, int i,
                                             const vec4_t<typename P::T>& pi, F&& f) {
     using T = typename P::T;
     using V = vec4_t<T>;
@@ -91,7 +92,7 @@ __device__ __forceinline__ void visit_group(const KParamsT<typename P::T>& k,
             T dx, dy, dz;
             rel_pos<P>(k, pi, a, P::kCodes ? slot_code(e) : 0u, dx, dy, dz);
             const T r2 = dist2(dx, dy, dz);
-            if (r2 < k.kh2) f(j, a, b, dx, dy, dz, r2);
+            if (inside(r2, k.kh2)) f(j, a, b, dx, dy, dz, r2, ld_vol(vol, j));
         };
         // this lane's chunks s, s + G, ... (each pair of lanes gathers two consecutive entries
         // per step)
@@ -135,10 +136,10 @@ __device__ __forceinline__ void visit_group(const KParamsT<typename P::T>& k,
                     T dx, dy2, dz2;
                     rel_pos<P>(k, pi, pj, code, dx, dy2, dz2);
                     const T r2 = dist2(dx, dy2, dz2);
-                    if (r2 < k.kh2 && j != i) {
+                    if (inside(r2, k.kh2) && j != i) {
                         V a, b;
                         ld_rec(R, j, a, b);
-                        f(j, a, b, dx, dy2, dz2, r2);
+                        f(j, a, b, dx, dy2, dz2, r2, ld_vol(vol, j));
                     }
                 }
             }
@@ -164,9 +165,10 @@ k_pass1_g(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         if (t < k.n) {
             const int i = work_slot(nl, t);
             acc.load(in.rec, i);
-            visit_group<P, G, 1>(k, cs, keys, nl, in.xyz, in.rec, t, i, acc.pi,
-                                 [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
-                acc.pair(k, aj, vj, dx, dy, dz, r2);
+            visit_group<P, G, 1>(k, cs, keys, nl, in.xyz, in.rec, in.vol, t, i, acc.pi,
+                                 [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2,
+                                     T vol) {
+                acc.pair(k, aj, vj, dx, dy, dz, r2, vol);
             });
         }
         reduce_group<G>(acc.dofv);

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "sph_internal.h"
 
 namespace sph {
@@ -187,6 +189,12 @@ __device__ __forceinline__ void pad_record(vec4_t<T>* R, int n) {
     R[2 * (size_t)n + 1] = make4<T>(T(0), T(0), T(0), T(-1));
 }
 
+// pair_volume of record j (FP64); nothing to load otherwise.
+__device__ __forceinline__ float ld_vol(const float*, int) { return 0.f; }
+__device__ __forceinline__ double ld_vol(const double* __restrict__ vol, int j) {
+    return __ldg(vol + j);
+}
+
 // Squared distance with an explicit rounding sequence, so the in-range test gives the same
 // answer in the list build, in the walking passes and in the list passes.
 __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
@@ -195,6 +203,18 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 __device__ __forceinline__ double dist2(double dx, double dy, double dz) {
     return __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
 }
+__device__ __forceinline__ bool fluid_rec(float signed_rho) { return signed_rho > 0.f; }
+// the same by integer instructions (FP64 comparisons run at the FP64 rate): positive, not NaN
+__device__ __forceinline__ bool fluid_rec(double signed_rho) {
+    return (unsigned)(__double2hiint(signed_rho) - 1) < 0x7ff00000u;
+}
+// r2 < cut2 of a squared distance (never negative; NaN is not inside)
+__device__ __forceinline__ bool inside(float r2, float cut2) { return r2 < cut2; }
+__device__ __forceinline__ bool inside(double r2, double cut2) {
+    return (unsigned long long)__double_as_longlong(r2) <
+           (unsigned long long)__double_as_longlong(cut2);
+}
+
 // Pair arithmetic: in FP32 the distance and the reciprocal of a pair come from the hardware's
 // approximate instructions (sqrt.approx, rcp.approx: within about one ulp, instead of the
 // correctly rounded sequences); FP64 keeps correctly rounded sqrt and division.  The .ftz
@@ -208,13 +228,31 @@ __device__ __forceinline__ float pair_sqrt(float x) {
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double pair_sqrt(double x) { return sqrt(x); }
+// FP64: the hardware's approximate reciprocal and reciprocal square root (about 20 bits, from the
+// upper word) refined by one third-order step of Householder's iteration, whose error is the cube of
+// the approximation's.  With y ~ 1/x and e = 1 - x y: 1/x = y (1 + e + e^2).  With y ~ x^(-1/2),
+// s = x y and the residual d = x - s^2 (exact in one fused operation): sqrt(x) = s + d y (1/2 +
+// 3 d y^2 / 8).  The last operation rounds a sum whose second term is small, so both end within
+// 0.5001 ulp, for three and six FP64 instructions.  The arguments are normal numbers far from the
+// ends of the range (r^2 + eta^2; r^2, which may be 0).
+__device__ __forceinline__ double pair_sqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    if (__double2hiint(x) < 0x00100000) y = 0.0;  // 0 (coincident particles): sqrt = 0
+    const double s = __dmul_rn(x, y), h = __dmul_rn(__fma_rn(-s, s, x), y);
+    return __fma_rn(h, __fma_rn(__dmul_rn(h, y), 0.375, 0.5), s);
+}
 __device__ __forceinline__ float pair_rcp(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double pair_rcp(double x) { return 1.0 / x; }
+__device__ __forceinline__ double pair_rcp(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-x, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
 __device__ __forceinline__ float dabs(float x) { return fabsf(x); }
 __device__ __forceinline__ double dabs(double x) { return fabs(x); }
 
@@ -518,13 +556,10 @@ __device__ __forceinline__ void walk_pairs(const KParamsT<typename P::T>& k,
         T dx, dy, dz;
         rel_pos<P>(k, pi, pj, code, dx, dy, dz);
         const T r2 = dist2(dx, dy, dz);
-        if (r2 < cut2 && j != i) f(j, code, pj, dx, dy, dz, r2);
+        if (inside(r2, cut2) && j != i) f(j, code, pj, dx, dy, dz, r2);
     });
 }
 
-
-template <class T>
-__device__ __forceinline__ bool fluid_rec(T signed_rho) { return signed_rho > T(0); }
 
 // Position the list build records for the displacement test (offsets in mixed precision).
 __device__ __forceinline__ float4 as_float4(const float4& v) { return v; }
@@ -581,11 +616,19 @@ struct Pass1Acc {
         vi = R[2 * (size_t)i + 1];
         fi = fluid_rec(vi.w);
     }
-    // One neighbour inside the support radius.
+    // One neighbour inside the support radius (record j; FP64: volj = c_fr mass / rho_j).
     __device__ __forceinline__ void pair(const KParamsT<T>& k, const V& aj, const V& vj, T dx,
-                                         T dy, T dz, T r2) {
+                                         T dy, T dz, T r2, T volj) {
         if (!fluid_rec(vj.w)) return;
         const T rr = pair_sqrt(r2);
+        if constexpr (std::is_same<T, double>::value) {
+            if (fi) {
+                const T t = fma_rn(T(-0.5) * k.inv_h, rr, T(1));
+                const T t3 = mul_rn(mul_rn(t, t), t);
+                dofv.add_prod(-mul_rn(t3, dot_rn(vi, vj, dx, dy, dz)), volj);
+                return;
+            }
+        }
         const T q = mul_rn(rr, k.inv_h);
         const T t = fma_rn(T(-0.5), q, T(1));
         const T t2 = mul_rn(t, t);
@@ -638,6 +681,7 @@ struct Pass1Acc {
         out.nrec[2 * (size_t)i] = make4<T>(pi.x, pi.y, pi.z, qv);
         out.nrec[2 * (size_t)i + 1] = make4<T>(vi.x, vi.y, vi.z, fi ? rho : -rho);
         out.self[i] = make4<T>(p, rho, dv, T(0));
+        if constexpr (std::is_same<T, double>::value) out.vol[i] = pair_volume(k, rho);
         if constexpr (WRITE_SUMS) {
             rhop_sum[i] = (float)rsum;
             w_sum[i] = (float)wsum;
@@ -677,18 +721,22 @@ struct Pass2Acc {
         damp_i = k.damper * si.z;
         active = fi || (MODE == MODE_RATES && wall_rates);
     }
-    // One neighbour inside the support radius.  aj = (x, y, z, q), vj = (vx, vy, vz, ±rho).
-    // rho_i - rho_j stays an exact difference of two close floats; writing the
-    // density-diffusion term with the volume m / rho_j instead (rho_i V_j - m) cancels and lost
-    // three digits of rho_dt.
+    // One neighbour inside the support radius.  aj = (x, y, z, q), vj = (vx, vy, vz, ±rho); FP64:
+    // volj = c_fr mass / rho_j.  rho_i - rho_j stays an exact difference of two close values;
+    // writing the density-diffusion term with the volume m / rho_j instead (rho_i V_j - m) cancels
+    // and lost three digits of rho_dt.
     __device__ __forceinline__ void pair(const KParamsT<T>& k, const Pass1OutT<T>& p1, int j,
-                                         const V& aj, const V& vj, T dx, T dy, T dz, T r2) {
+                                         const V& aj, const V& vj, T dx, T dy, T dz, T r2, T volj) {
         const bool fj = fluid_rec(vj.w);
         const T rhoj = dabs(vj.w);
         const T rr = pair_sqrt(r2);
         const T t = fma_rn(mul_rn(T(-0.5), k.inv_h), rr, T(1));
         // m / rho_j grad W / r in one factor: c_fr m t^3 / rho_j
-        const T w = mul_rn(mul_rn(mul_rn(k.c_fr_mass, mul_rn(t, t)), t), pair_rcp(rhoj));
+        T w;
+        if constexpr (std::is_same<T, double>::value)
+            w = mul_rn(mul_rn(mul_rn(t, t), t), volj);
+        else
+            w = mul_rn(mul_rn(mul_rn(k.c_fr_mass, mul_rn(t, t)), t), pair_rcp(rhoj));
         const T vdotr = dot_rn(vi, vj, dx, dy, dz);
         const T inv_r2e = pair_rcp(add_rn(r2, k.eta2));
         const T diff = mul_rn(mul_rn(mul_rn(sub_rn(rhoi, rhoj), k.delta_h_cs), r2), inv_r2e);
@@ -916,6 +964,7 @@ __device__ __forceinline__ void pass2_finish(const KParamsT<typename P::T>& k, i
             tp = make4<T>(pi.x, pi.y, pi.z, rhoi);
             tv = make4<T>(vi.x, vi.y, vi.z, T(0));
         }
+        if constexpr (std::is_same<T, double>::value) out.vol[i] = pair_volume(k, nrho);
         out.rec[2 * (size_t)i] = make4<T>(np.x, np.y, np.z, npres);
         out.rec[2 * (size_t)i + 1] = make4<T>(nv.x, nv.y, nv.z, fi ? nrho : -nrho);
         if (out.xyz) out.xyz[i] = make4<T>(np.x, np.y, np.z, fi ? T(1) : T(-1));

@@ -272,10 +272,10 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
                 float dx, dy, dz;
                 rel_pos<P>(k, A.pi, aj, 0u, dx, dy, dz);
                 float r2 = dist2(dx, dy, dz);
-                if (!A.fi && r2 < k.kh2) A.pair(k, aj, vj, dx, dy, dz, r2);
+                if (!A.fi && r2 < k.kh2) A.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
                 rel_pos<P>(k, B.pi, aj, 0u, dx, dy, dz);
                 r2 = dist2(dx, dy, dz);
-                if (!B.fi && r2 < k.kh2) B.pair(k, aj, vj, dx, dy, dz, r2);
+                if (!B.fi && r2 < k.kh2) B.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
             });
         }
     } else {
@@ -287,7 +287,7 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
                                  float r2) {
                 float4 aj, vj;
                 ld_rec(in.rec, j, aj, vj);
-                C.pair(k, aj, vj, dx, dy, dz, r2);
+                C.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
             });
             if (m) B = C;
             else A = C;
@@ -325,7 +325,7 @@ k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
                                              float dz, float r2) {
                             float4 aj, vj;
                             ld_rec(p1.nrec, j, aj, vj);
-                            C.pair(k, p1, j, aj, vj, dx, dy, dz, r2);
+                            C.pair(k, p1, j, aj, vj, dx, dy, dz, r2, 0.f);
                         });
                     if (m) B = C;
                     else A = C;

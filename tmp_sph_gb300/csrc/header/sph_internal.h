@@ -102,6 +102,12 @@ __device__ __forceinline__ float3 record_pos(const KParamsT<KT>& k, unsigned key
         return make_float3((float)x, (float)y, (float)z);
     }
 }
+// FP64 runs at 1/64 of the FP32 rate and bounds the FP64 passes, so what a pair needs of its
+// neighbour's density is divided out once per particle: c_fr mass / rho, kept beside the records.
+template <class T>
+__device__ __forceinline__ T pair_volume(const KParamsT<T>& k, T rho) {
+    return k.c_fr_mass / rho;
+}
 // The list slots carry a cell code above a 26-bit neighbour index.
 inline bool prec_has_codes(int prec) {
     return prec == SPH_PREC_MIXED || prec == SPH_PREC_MIXED_COMP;
@@ -128,6 +134,7 @@ struct ParticleSetT {
     dvec4* xm = nullptr;
     dvec4* txm = nullptr;
     int* inst = nullptr;  // batched instances: the particle's instance (0 for one simulation)
+    T* vol = nullptr;  // FP64: c_fr mass / rho of every record (NULL otherwise)
 };
 using ParticleSet = ParticleSetT<float>;
 
@@ -138,6 +145,7 @@ template <class T>
 struct Pass1OutT {
     vec4_t<T>* nrec = nullptr;
     vec4_t<T>* self = nullptr;
+    T* vol = nullptr;  // FP64: c_fr mass / rho' of every record (NULL otherwise)
 };
 using Pass1Out = Pass1OutT<float>;
 

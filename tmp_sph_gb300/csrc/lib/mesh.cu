@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "sph_internal.h"
 
@@ -425,6 +426,7 @@ __global__ void k_gather(KParamsT<typename P::T> kp, const int* __restrict__ per
     dst.id[k] = src.id[s];
     if (src.inst && dst.inst) dst.inst[k] = src.inst[s];
     if (with_tmp) dst.tvel[k] = src.tvel[s];
+    if constexpr (std::is_same<T, double>::value) dst.vol[k] = src.vol[s];
 }
 
 // ---------------------------------------------------------------- work order
@@ -584,6 +586,7 @@ __global__ void k_upload_convert(KParamsT<typename P::T> kp, const float* __rest
     } else {
         dst.rec[2 * (size_t)i] = make4<T>(x, y, z, (T)p[i]);
         dst.tpos[i] = make4<T>(x, y, z, (T)rho[i]);
+        if constexpr (std::is_same<T, double>::value) dst.vol[i] = pair_volume(kp, (T)rho[i]);
         hash[i] = slot_key(kp, inst, t == SPH_TYPE_FLUID, (T)x, (T)y, (T)z, &f);
     }
     raise_flags(err, f);
@@ -634,6 +637,8 @@ __global__ void k_upload_sorted(KParamsT<typename P::T> kp, const float* __restr
             } else {
                 a = make4<T>(x, y, z, (T)p[r]);
                 dst.tpos[k] = make4<T>(x, y, z, (T)rho[r]);
+                if constexpr (std::is_same<T, double>::value)
+                    dst.vol[k] = pair_volume(kp, (T)rho[r]);
                 nk = slot_key(kp, inst, t == SPH_TYPE_FLUID, (T)x, (T)y, (T)z, &f);
             }
             hash[k] = nk;

@@ -29,6 +29,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "sph_internal.h"
@@ -46,6 +47,7 @@ template <class T>
 void free_set(ParticleSetT<T>& s) {
     cudaFree(s.rec); cudaFree(s.xyz); cudaFree(s.type); cudaFree(s.id);
     cudaFree(s.tpos); cudaFree(s.tvel); cudaFree(s.xm); cudaFree(s.txm); cudaFree(s.inst);
+    cudaFree(s.vol);
     s = ParticleSetT<T>{};
 }
 
@@ -59,6 +61,7 @@ cudaError_t alloc_set(ParticleSetT<T>& s, int cap, bool mixed) {
     if ((e = dalloc(&s.tpos, cap)) != cudaSuccess) return e;
     if ((e = dalloc(&s.tvel, cap)) != cudaSuccess) return e;
     if ((e = dalloc(&s.inst, cap)) != cudaSuccess) return e;
+    if (std::is_same<T, double>::value && (e = dalloc(&s.vol, (size_t)cap + 1)) != cudaSuccess) return e;
     if (mixed) {
         if ((e = dalloc(&s.xm, cap)) != cudaSuccess) return e;
         if ((e = dalloc(&s.txm, cap)) != cudaSuccess) return e;
@@ -70,6 +73,7 @@ template <class T>
 void free_p1(Pass1OutT<T>& p) {
     cudaFree(p.nrec);
     cudaFree(p.self);
+    cudaFree(p.vol);
     p = Pass1OutT<T>{};
 }
 
@@ -77,6 +81,7 @@ template <class T>
 cudaError_t alloc_p1(Pass1OutT<T>& p, int cap) {
     cudaError_t e = dalloc(&p.nrec, 2 * ((size_t)cap + 1));
     if (e == cudaSuccess) e = dalloc(&p.self, cap);
+    if (e == cudaSuccess && std::is_same<T, double>::value) e = dalloc(&p.vol, (size_t)cap + 1);
     return e;
 }
 
@@ -304,12 +309,16 @@ constexpr bool kTwin = P::kId == SPH_PREC_FP32 || P::kId == SPH_PREC_MIXED_ABS;
 
 // Threads per block of the neighbour kernels: the option, or by default 64 with two particles per
 // thread (104 registers a thread: nine blocks per SM; 128 threads: pass 2 596 against 582 us at
-// 4.96M particles), else 256 in FP32 (their static shared memory is sized for 256 threads) and 128
-// in the other precisions.
+// 4.96M particles), 32 in FP64 (its pipe bounds a pass, so the SMs should get equal shares of warps:
+// 133,968 particles, three steps 6.56 ms with 128, 6.28 with 32; 27,288 particles 3.29 and 2.97),
+// else 256 in FP32 up to 60,000 particles and 128 above, where whole blocks of 256 leave SMs
+// unequal shares (133,968 particles, ten steps 1.23 ms with 256, 1.15 with 128; level at 380,000),
+// and 128 in mixed precision on cell-local offsets.
 static int block_threads(const sph_ctx* c) {
     if (c->opt_threads > 0) return c->opt_threads;
     if (twin_lists(c)) return 64;
-    return fp32_pairs(c->prec) ? 256 : 128;
+    if (c->prec == SPH_PREC_FP64) return 32;
+    return !fp32_pairs(c->prec) || c->n >= 60000 ? 128 : 256;
 }
 
 // Cells per list cutoff by default: 3 in FP32 (cells of about dx at h = 1.3 dx: the
