@@ -6,8 +6,7 @@
 // recoverD/recover (src/lib/mesh.cu:162-194).
 //
 // The sort is written for this project: reduce-then-scan LSD radix with 8-bit digits,
-// 4096-key tiles (256 threads x 16 keys), warp-level stable ranking with __match_any_sync,
-// tile-local reordering in shared memory so the scatter to global memory is in digit runs.
+// 4096-key tiles (512 threads x 8 keys), warp-level stable ranking with votes, tile-local reordering in shared memory so the scatter to global memory is in digit runs.
 // No spin-waits, no allocation: all scratch is caller-provided.
 #include <cuda_runtime.h>
 
@@ -20,9 +19,11 @@ namespace sph {
 
 namespace {
 
-constexpr int RS_THREADS = 256;
+// 512 threads x 8 keys: 2.1M random keys, upsweep / downsweep of a pass 11 / 21 us (256 x 16: 14 /
+// 27, too few warps for the latency of a tile; 1024 x 4: 11 / 26).
+constexpr int RS_THREADS = 512;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_IPT = 16;
+constexpr int RS_IPT = 8;
 constexpr int RS_TILE = RS_THREADS * RS_IPT;  // 4096 keys
 constexpr int RS_RADIX = 256;
 constexpr int RS_MAX_PASSES = 4;
@@ -57,6 +58,22 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
+// Lanes of the warp with the same 8-bit digit (valid lanes only; an invalid lane matches none of
+// them): one vote per bit.  __match_any_sync gives the same mask at about 70 cycles per SM and
+// call, which bound the sort at millions of keys (4.96M keys, a pass with 256 x 16 keys: upsweep 41
+// -> 25 us, downsweep 69 -> 53).
+__device__ __forceinline__ unsigned digit_peers(unsigned d, bool valid) {
+    unsigned peers = __ballot_sync(0xffffffffu, valid);
+    if (!valid) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        const bool bit = (d >> b) & 1u;
+        const unsigned v = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? v : ~v;
+    }
+    return peers;
+}
+
 // Per-tile digit histogram: hist[d * tiles + tile]; totals[d] accumulates over tiles.
 __global__ void __launch_bounds__(RS_THREADS)
 k_rs_upsweep(const unsigned* __restrict__ keys, int n, int shift, unsigned xmask,
@@ -65,7 +82,7 @@ k_rs_upsweep(const unsigned* __restrict__ keys, int n, int shift, unsigned xmask
     __shared__ unsigned cnt[RS_RADIX];
     if (gated_off(gate)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    cnt[tid] = 0;
+    if (tid < RS_RADIX) cnt[tid] = 0;
     __syncthreads();
     const long base = (long)blockIdx.x * RS_TILE + warp * (32 * RS_IPT) + lane;
     unsigned flags = 0;
@@ -76,22 +93,26 @@ k_rs_upsweep(const unsigned* __restrict__ keys, int n, int shift, unsigned xmask
         unsigned key = valid ? (__ldg(keys + idx) ^ xmask) : 0u;
         if (valid && check_bits < 32 && (key >> check_bits) != 0u) flags |= SPH_FLAG_KEY_RANGE;
         unsigned d = (key >> shift) & 0xffu;
-        unsigned peers = __match_any_sync(0xffffffffu, valid ? d : 0x100u);
+        unsigned peers = digit_peers(d, valid);
         if (valid && lane == __ffs(peers) - 1) atomicAdd(&cnt[d], __popc(peers));
     }
     __syncthreads();
-    unsigned c = cnt[tid];
-    hist[(size_t)tid * tiles + blockIdx.x] = c;
-    if (c) atomicAdd(&totals[tid], c);
+    if (tid < RS_RADIX) {
+        const unsigned c = cnt[tid];
+        hist[(size_t)tid * tiles + blockIdx.x] = c;
+        if (c) atomicAdd(&totals[tid], c);
+    }
     raise_flags(err, flags);
 }
 
+constexpr int SC_THREADS = 256;
+
 // Exclusive scan of one digit's row of tile counts, offset by the counts of all smaller
 // digits: after this, hist[d * tiles + t] is the first output slot of digit d in tile t.
-__global__ void __launch_bounds__(RS_THREADS)
+__global__ void __launch_bounds__(SC_THREADS)
 k_rs_scan(unsigned* __restrict__ hist, int tiles, const unsigned* __restrict__ totals,
           const unsigned* gate) {
-    __shared__ unsigned wsum[RS_WARPS];
+    __shared__ unsigned wsum[(SC_THREADS / 32)];
     __shared__ unsigned s_carry;
     if (gated_off(gate)) return;
     const int d = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -103,12 +124,12 @@ k_rs_scan(unsigned* __restrict__ hist, int tiles, const unsigned* __restrict__ t
     __syncthreads();
     if (tid == 0) {
         unsigned b = 0;
-        for (int w = 0; w < RS_WARPS; w++) b += wsum[w];
+        for (int w = 0; w < (SC_THREADS / 32); w++) b += wsum[w];
         s_carry = b;
     }
     __syncthreads();
     unsigned* row = hist + (size_t)d * tiles;
-    for (int chunk = 0; chunk < tiles; chunk += RS_THREADS) {
+    for (int chunk = 0; chunk < tiles; chunk += SC_THREADS) {
         int idx = chunk + tid;
         unsigned x = idx < tiles ? row[idx] : 0u;
         unsigned incl = x;
@@ -121,7 +142,7 @@ k_rs_scan(unsigned* __restrict__ hist, int tiles, const unsigned* __restrict__ t
         if (lane == 31) wsum[warp] = incl;
         __syncthreads();
         unsigned wpre = 0, btot = 0;
-        for (int w = 0; w < RS_WARPS; w++) {
+        for (int w = 0; w < (SC_THREADS / 32); w++) {
             unsigned t = wsum[w];
             if (w < warp) wpre += t;
             btot += t;
@@ -140,17 +161,18 @@ k_rs_downsweep(const unsigned* __restrict__ keys_in, const int* __restrict__ val
                unsigned* __restrict__ keys_out, int* __restrict__ vals_out,
                const unsigned* __restrict__ hist, int n, int shift, unsigned xmask_in,
                unsigned xmask_out, int tiles, const unsigned* gate) {
-    __shared__ unsigned s_cnt[RS_WARPS][RS_RADIX];
+    __shared__ unsigned short s_cnt[RS_WARPS][RS_RADIX];  // a tile holds 4096 keys
     __shared__ unsigned s_gbase[RS_RADIX];
     __shared__ unsigned s_tpre[RS_RADIX];
     __shared__ unsigned s_keys[RS_TILE];
     __shared__ int s_vals[RS_TILE];
-    __shared__ unsigned s_wsum[RS_WARPS];
+    __shared__ unsigned s_wsum[RS_RADIX / 32];
 
     if (gated_off(gate)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < RS_RADIX)
 #pragma unroll
-    for (int w = 0; w < RS_WARPS; w++) s_cnt[w][tid] = 0;
+        for (int w = 0; w < RS_WARPS; w++) s_cnt[w][tid] = 0;
     __syncthreads();
 
     const long tile_base = (long)blockIdx.x * RS_TILE;
@@ -170,35 +192,39 @@ k_rs_downsweep(const unsigned* __restrict__ keys_in, const int* __restrict__ val
     for (int r = 0; r < RS_IPT; r++) {
         bool valid = wbase + r * 32 < n;
         unsigned d = (key[r] >> shift) & 0xffu;
-        unsigned peers = __match_any_sync(0xffffffffu, valid ? d : 0x100u);
+        unsigned peers = digit_peers(d, valid);
         unsigned c = valid ? s_cnt[warp][d] : 0u;
         __syncwarp();
-        if (valid && lane == __ffs(peers) - 1) s_cnt[warp][d] = c + __popc(peers);
+        if (valid && lane == __ffs(peers) - 1) s_cnt[warp][d] = (unsigned short)(c + __popc(peers));
         __syncwarp();
         lr[r] = c + __popc(peers & lt);
     }
     __syncthreads();
-    // per digit: exclusive prefix over warps, tile count, global base
-    unsigned run = 0;
+    // per digit (the first 256 threads): exclusive prefix over warps, tile count, global base
+    unsigned run = 0, incl = 0;
+    if (tid < RS_RADIX) {
 #pragma unroll
-    for (int w = 0; w < RS_WARPS; w++) {
-        unsigned v = s_cnt[w][tid];
-        s_cnt[w][tid] = run;
-        run += v;
-    }
-    s_gbase[tid] = hist[(size_t)tid * tiles + blockIdx.x];
-    // exclusive scan of tile counts over digits
-    unsigned incl = run;
+        for (int w = 0; w < RS_WARPS; w++) {
+            const unsigned v = s_cnt[w][tid];
+            s_cnt[w][tid] = (unsigned short)run;
+            run += v;
+        }
+        s_gbase[tid] = hist[(size_t)tid * tiles + blockIdx.x];
+        // exclusive scan of tile counts over digits
+        incl = run;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_wsum[warp] = incl;
     }
-    if (lane == 31) s_wsum[warp] = incl;
     __syncthreads();
-    unsigned wpre = 0;
-    for (int w = 0; w < warp; w++) wpre += s_wsum[w];
-    s_tpre[tid] = wpre + incl - run;
+    if (tid < RS_RADIX) {
+        unsigned wpre = 0;
+        for (int w = 0; w < warp; w++) wpre += s_wsum[w];
+        s_tpre[tid] = wpre + incl - run;
+    }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < RS_IPT; r++) {
@@ -851,7 +877,7 @@ cudaError_t radix_sort_pairs(const unsigned* keys_in, const int* vals_in, unsign
         unsigned* totals = sc.totals + (size_t)p * RS_RADIX;
         k_rs_upsweep<<<tiles, RS_THREADS, 0, s>>>(kin, n, shift, xin, p == 0 ? key_bits : 32,
                                                    sc.hist, tiles, totals, err, gate);
-        k_rs_scan<<<RS_RADIX, RS_THREADS, 0, s>>>(sc.hist, tiles, totals, gate);
+        k_rs_scan<<<RS_RADIX, SC_THREADS, 0, s>>>(sc.hist, tiles, totals, gate);
         k_rs_downsweep<<<tiles, RS_THREADS, 0, s>>>(kin, vin, kdst, vdst, sc.hist, n, shift, xin,
                                                      xout, tiles, gate);
         kin = kdst;
