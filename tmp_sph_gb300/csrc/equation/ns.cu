@@ -270,7 +270,10 @@ __device__ __forceinline__ void pass1_one(const KParamsT<typename P::T>& k,
     const int i = work_slot(nl, t);
     Pass1Acc<P> acc;
     acc.load(in.rec, i);
-    visit_records<P, LIST, 1>(k, cs, keys, nl, in.xyz, in.rec, in.vol, t, i, acc,
+    // a particle whose list overflowed walks the records' positions, a pass without lists the dense
+    // ones of this half step's rebuild
+    visit_records<P, LIST, LIST == LIST_NONE ? 1 : 2>(k, cs, keys, nl,
+                              LIST == LIST_NONE ? in.xyz : in.rec, in.rec, in.vol, t, i, acc,
                               [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2, T vol) {
         acc.pair(k, aj, vj, dx, dy, dz, r2, vol);
     });

@@ -165,7 +165,7 @@ k_pass1_g(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         if (t < k.n) {
             const int i = work_slot(nl, t);
             acc.load(in.rec, i);
-            visit_group<P, G, 1>(k, cs, keys, nl, in.xyz, in.rec, in.vol, t, i, acc.pi,
+            visit_group<P, G, 2>(k, cs, keys, nl, in.rec, in.rec, in.vol, t, i, acc.pi,
                                  [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2,
                                      T vol) {
                 acc.pair(k, aj, vj, dx, dy, dz, r2, vol);

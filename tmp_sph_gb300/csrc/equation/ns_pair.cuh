@@ -697,9 +697,9 @@ enum { MODE_RATES = 0, MODE_PRED = 1, MODE_CORR = 2 };
 // midpoint predictor / corrector of src/sph/sph_run.cu:425-519 is applied and the updated
 // particle written to `out` with its next cell hash.
 //
-// `out` may alias `in`: the update touches only particle i's own rows, and neighbours (also
-// the positions of a cell walk) come from the pass-1 records.  Returns the squared distance
-// of particle i from its position when the neighbour list was built (0 without a list).
+// `out` is `in`, updated in place: the update touches only particle i's own rows, neighbours (also
+// the positions of a cell walk) come from the pass-1 records, and kind, id and instance stay.  The
+// dense positions (xyz) are those of the last rebuild: only a rebuild reads them.
 // Pass-2 state of one particle: its pass-1 record, own side and the four neighbour sums.
 template <class P, int MODE>
 struct Pass2Acc {
@@ -879,9 +879,6 @@ __device__ __forceinline__ void pass2_finish(const KParamsT<typename P::T>& k, i
         const float px = q.x, py = q.y, pz = q.z;
         out.rec[2 * (size_t)i] = make_float4(px, py, pz, npres);
         out.rec[2 * (size_t)i + 1] = make_float4(nv.x, nv.y, nv.z, fi ? nrho : -nrho);
-        if (out.xyz) out.xyz[i] = make_float4(px, py, pz, fi ? 1.f : -1.f);
-        out.type[i] = in.type[i];
-        out.id[i] = in.id[i];
         out.xm[i] = nxm;
         if (MODE == MODE_PRED) {
             out.txm[i] = txm;
@@ -889,7 +886,6 @@ __device__ __forceinline__ void pass2_finish(const KParamsT<typename P::T>& k, i
         }
         // instance ids only move with the particles when instances are batched
         const int inst = k.inst_cells ? in.inst[i] : 0;
-        if (k.inst_cells) out.inst[i] = inst;
         unsigned f = 0;
         const unsigned nk = P::kCodes ? slot_key(k, inst, fi, nxm.x, nxm.y, nxm.z, &f)
                                        : slot_key(k, inst, fi, px, py, pz, &f);
@@ -967,16 +963,12 @@ __device__ __forceinline__ void pass2_finish(const KParamsT<typename P::T>& k, i
         if constexpr (std::is_same<T, double>::value) out.vol[i] = pair_volume(k, nrho);
         out.rec[2 * (size_t)i] = make4<T>(np.x, np.y, np.z, npres);
         out.rec[2 * (size_t)i + 1] = make4<T>(nv.x, nv.y, nv.z, fi ? nrho : -nrho);
-        if (out.xyz) out.xyz[i] = make4<T>(np.x, np.y, np.z, fi ? T(1) : T(-1));
-        out.type[i] = in.type[i];
-        out.id[i] = in.id[i];
         if (MODE == MODE_PRED) {
             out.tpos[i] = tp;
             out.tvel[i] = tv;
         }
         // instance ids only move with the particles when instances are batched
         const int inst = k.inst_cells ? in.inst[i] : 0;
-        if (k.inst_cells) out.inst[i] = inst;
         unsigned f = 0;
         const unsigned nk = slot_key(k, inst, fi, np.x, np.y, np.z, &f);
         out_hash[i] = nk;

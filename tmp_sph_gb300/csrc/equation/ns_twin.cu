@@ -421,7 +421,7 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
 #pragma unroll 1
         for (int m = 0; m < 2; m++) {
             Pass1Acc<P> C = m ? B : A;
-            walk_pairs<P, 1>(k, cs, keys, in.xyz, m ? tw.b : tw.a, C.pi, k.kh2,
+            walk_pairs<P, 2>(k, cs, keys, in.rec, m ? tw.b : tw.a, C.pi, k.kh2,
                              [&](int j, unsigned, const float4&, float dx, float dy, float dz,
                                  float r2) {
                 float4 aj, vj;

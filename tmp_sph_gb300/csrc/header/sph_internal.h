@@ -126,7 +126,8 @@ inline bool prec_has_codes(int prec) {
 template <class T>
 struct ParticleSetT {
     vec4_t<T>* rec = nullptr;
-    vec4_t<T>* xyz = nullptr;  // sorted set only: dense (x, y, z, ±1) for candidate walks
+    vec4_t<T>* xyz = nullptr;  // sorted set only: dense (x, y, z, ±1) at the last rebuild, for the
+                               // list build and the passes that walk the cells after every one
     int* type = nullptr;
     int* id = nullptr;
     vec4_t<T>* tpos = nullptr;
@@ -211,7 +212,7 @@ cudaError_t launch_pass2_rates(const KParams& k, const ParticleSet& in,
                                const unsigned* sorted_keys, const int* cell_start,
                                const NbrList* nl, const Pass1Out& p1, float* rho_dt,
                                float* vel_dt, int wall_rates, cudaStream_t s);
-// `out` may be `in` (the update is per particle; neighbours are read from p1).  disp (may be
+// `out` is `in` (the update is per particle; neighbours are read from p1).  disp (may be
 // NULL) receives, by atomicMax on its float bits, the largest squared distance of a fluid
 // particle from its position when the list was built (nl->xb).
 template <class P>
@@ -241,6 +242,7 @@ cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet
 // Resident-state glue (lib/mesh.cu), one instantiation per precision policy P.
 // perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
 // cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).
+// with_tmp: also the predictor's saved state; dense: also dst.xyz.
 // The work order of the list kernels (NbrList::order) of a cell-sorted set on `grid`: its fluid
 // slots, then the others, each in slot order or (rows) with pairs of rows merged so that
 // consecutive positions hold particles one above the other.  Scratch: rank (n + 1 ints) and
@@ -251,7 +253,7 @@ cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int
 template <class P>
 cudaError_t launch_gather(const KParamsT<typename P::T>& k, const int* perm,
                           const ParticleSetT<typename P::T>& src, ParticleSetT<typename P::T> dst,
-                          int with_tmp, const unsigned* keys, cudaStream_t s,
+                          int with_tmp, int dense, const unsigned* keys, cudaStream_t s,
                           const unsigned* gate = nullptr);
 // Recompute the cell keys of `set` on the grid of `k` (k.n particles).
 template <class P>

@@ -503,12 +503,16 @@ __device__ __forceinline__ float4 offsets_in_cell(const KParamsT<KT>& k, unsigne
     return make_float4(q.x, q.y, q.z, w);
 }
 
-// Permute (perm) or copy (perm == NULL) a particle set.  With cell codes a permuting gather
-// re-expresses positions as offsets in the new cells keys[k].
+// Permute (perm) or copy (perm == NULL) a particle set.  with_tmp: the predictor's saved state too
+// (it holds nothing between a corrector and the next predictor).  dense: write dst.xyz as well (the
+// scratch set needs none).  With cell codes a permuting gather re-expresses positions as offsets in
+// the new cells keys[k].  Bound by DRAM: the copies of a rebuild at 4.96M particles took 2 x 128 us
+// with every array moved each time, 70 + 74 now before a predictor.
 template <class P>
 __global__ void k_gather(KParamsT<typename P::T> kp, const int* __restrict__ perm,
                          ParticleSetT<typename P::T> src, ParticleSetT<typename P::T> dst,
-                         int with_tmp, const unsigned* __restrict__ keys, const unsigned* gate) {
+                         int with_tmp, int dense, const unsigned* __restrict__ keys,
+                         const unsigned* gate) {
     using T = typename P::T;
     using V = vec4_t<T>;
     if (gated_off(gate)) return;
@@ -530,10 +534,10 @@ __global__ void k_gather(KParamsT<typename P::T> kp, const int* __restrict__ per
     }
     dst.rec[2 * (size_t)k] = a;
     dst.rec[2 * (size_t)k + 1] = b;
-    dst.xyz[k] = make4<T>(a.x, a.y, a.z, b.w > T(0) ? T(1) : T(-1));
+    if (dense) dst.xyz[k] = make4<T>(a.x, a.y, a.z, b.w > T(0) ? T(1) : T(-1));
     dst.type[k] = src.type[s];
     dst.id[k] = src.id[s];
-    if (src.inst && dst.inst) dst.inst[k] = src.inst[s];
+    if (kp.inst_cells) dst.inst[k] = src.inst[s];
     if (with_tmp) dst.tvel[k] = src.tvel[s];
     if constexpr (std::is_same<T, double>::value) dst.vol[k] = src.vol[s];
 }
@@ -763,7 +767,6 @@ __global__ void k_upload_sorted(KParamsT<typename P::T> kp, const float* __restr
                 box.add_at(iw, inst, -3.0e38f, -3.0e38f, -3.0e38f);
             }
             dst.rec[2 * (size_t)k] = a;
-            dst.xyz[k] = make4<T>(a.x, a.y, a.z, srho > T(0) ? T(1) : T(-1));
             raise_flags(err, f);
             if (xb && !out_now && !moved_out) {
                 const float4 b = xb[k];
@@ -792,7 +795,7 @@ __global__ void k_rehash(KParamsT<typename P::T> kp, ParticleSetT<typename P::T>
         const dvec4 q = set.xm[i];
         hash[i] = slot_key(kp, inst, fluid, q.x, q.y, q.z, &f);
     } else {
-        const auto q = set.xyz[i];
+        const auto q = set.rec[2 * (size_t)i];
         hash[i] = slot_key(kp, inst, fluid, q.x, q.y, q.z, &f);
     }
     raise_flags(err, f);
@@ -972,14 +975,14 @@ cudaError_t radix_sort_pairs(const unsigned* keys_in, const int* vals_in, unsign
 cudaError_t build_cell_starts(const unsigned* sorted_keys, int n, int num_cells, int* cs,
                               cudaStream_t s, const unsigned* gate, const int* type,
                               unsigned char* fluid_cells) {
-    cudaError_t e = fill_u32(reinterpret_cast<unsigned*>(cs), 0x7f7f7f7fu, (long)num_cells + 1,
-                             gate, s);
-    if (e != cudaSuccess) return e;
     if (num_cells >= n) {
         k_cell_starts<<<blocks_for((long)num_cells + 1, CS_CELLS), CS_THREADS, 0, s>>>(
             sorted_keys, n, num_cells, cs, type, type ? fluid_cells : nullptr, gate);
         return cudaGetLastError();
     }
+    cudaError_t e = fill_u32(reinterpret_cast<unsigned*>(cs), 0x7f7f7f7fu, (long)num_cells + 1,
+                             gate, s);
+    if (e != cudaSuccess) return e;
     if (fluid_cells && type) {
         e = fill_u32(reinterpret_cast<unsigned*>(fluid_cells), 0u, ((long)num_cells + 4) / 4,
                      gate, s);
@@ -1012,11 +1015,12 @@ cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int
 template <class P>
 cudaError_t launch_gather(const KParamsT<typename P::T>& k, const int* perm,
                           const ParticleSetT<typename P::T>& src, ParticleSetT<typename P::T> dst,
-                          int with_tmp, const unsigned* keys, cudaStream_t s,
+                          int with_tmp, int dense, const unsigned* keys, cudaStream_t s,
                           const unsigned* gate) {
     if (k.n <= 0) return cudaSuccess;
     if (P::kCodes && perm && !keys) return cudaErrorInvalidValue;
-    k_gather<P><<<blocks_for(k.n, 256), 256, 0, s>>>(k, perm, src, dst, with_tmp, keys, gate);
+    k_gather<P><<<blocks_for(k.n, 256), 256, 0, s>>>(k, perm, src, dst, with_tmp, dense, keys,
+                                                     gate);
     return cudaGetLastError();
 }
 
@@ -1077,7 +1081,7 @@ cudaError_t launch_download_f64(const KParamsT<typename P::T>& k,
                                                 cudaStream_t);                                  \
     template cudaError_t launch_gather<P>(const KParamsT<P::T>&, const int*,                    \
                                           const ParticleSetT<P::T>&, ParticleSetT<P::T>, int,   \
-                                          const unsigned*, cudaStream_t, const unsigned*);      \
+                                          int, const unsigned*, cudaStream_t, const unsigned*); \
     template cudaError_t launch_upload_convert<P>(const KParamsT<P::T>&, const float*,          \
                                                   const float*, const float*, const float*,     \
                                                   const int*, const int*, int,                  \

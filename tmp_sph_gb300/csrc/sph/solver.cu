@@ -569,8 +569,8 @@ struct CondCapture {
 
 // Sort, gather, cell starts and list build, each kernel gated on rb[0].  `ev` as half_step.
 template <class P>
-cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, cudaStream_t s,
-                          cudaEvent_t* ev) {
+cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, HalfStep half,
+                          cudaStream_t s, cudaEvent_t* ev) {
     // with park_inactive, key num_cells marks the slots outside the neighbour search
     const int bits = key_bits_for(c->Pi.num_cells + (c->P.park_inactive ? 1 : 0));
     const NbrList* nl = list_for(c);
@@ -588,9 +588,11 @@ cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, cudaStre
     // permute the live set y into cell order through x, then copy it back
     auto& x = State<P>::x(c);
     auto& y = State<P>::y(c);
-    if ((e = launch_gather<P>(k, c->perm, y, x, 1, c->keys_sorted, s, gate)) != cudaSuccess)
+    // (the predictor's saved state only between a predictor and its corrector)
+    const int tmp = half == HALF_CORRECT ? 1 : 0;
+    if ((e = launch_gather<P>(k, c->perm, y, x, tmp, 0, c->keys_sorted, s, gate)) != cudaSuccess)
         return e;
-    if ((e = launch_gather<P>(k, nullptr, x, y, 1, nullptr, s, gate)) != cudaSuccess) return e;
+    if ((e = launch_gather<P>(k, nullptr, x, y, tmp, 1, nullptr, s, gate)) != cudaSuccess) return e;
     if ((e = build_cell_starts(c->keys_sorted, c->n, c->Pi.num_cells, c->cell_start, s, gate,
                                y.type, c->fluid_cells)) !=
         cudaSuccess)
@@ -617,7 +619,7 @@ cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, cudaStre
 // captures the rebuild kernels into its body on cc.side.
 template <class P>
 cudaError_t capture_conditional_rebuild(sph_ctx* c, const KParamsT<typename P::T>& k,
-                                        cudaStream_t s, const CondCapture& cc) {
+                                        HalfStep half, cudaStream_t s, const CondCapture& cc) {
     cudaStreamCaptureStatus st;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -639,7 +641,7 @@ cudaError_t capture_conditional_rebuild(sph_ctx* c, const KParamsT<typename P::T
     if ((e = cudaStreamBeginCaptureToGraph(cc.side, body, nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return e;
-    e = rebuild_lists<P>(c, k, cc.side, nullptr);
+    e = rebuild_lists<P>(c, k, half, cc.side, nullptr);
     cudaGraph_t out = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(cc.side, &out);
     return e != cudaSuccess ? e : e2;
@@ -662,7 +664,8 @@ cudaError_t half_step(sph_ctx* c, HalfStep half, cudaStream_t s, cudaEvent_t* ev
     else
         k_decide<<<1, 1, 0, s>>>(c->rb, skin_control(c), nl ? 0 : 1, cc ? cc->handle : 0,
                                  cc ? 1 : 0);
-    e = cc ? capture_conditional_rebuild<P>(c, k, s, *cc) : rebuild_lists<P>(c, k, s, ev);
+    e = cc ? capture_conditional_rebuild<P>(c, k, half, s, *cc)
+           : rebuild_lists<P>(c, k, half, s, ev);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[PH_PASS1], s);
     if constexpr (kTwin<P>) {
