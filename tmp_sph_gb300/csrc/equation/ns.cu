@@ -165,19 +165,11 @@ __device__ __forceinline__ void nbr_build_one(const KParamsT<typename P::T>& k,
     const vec4_t<T> pi = X[i];
     if (nl.xb) nl.xb[i] = as_float4(pi);
     const bool keep_all = fluid_rec(pi.w) || walls_all;
-    if (!keep_all && nl.fluid_cells && !inactive_key(k, keys[i])) {
+    if (!keep_all && nl.rank && !inactive_key(k, keys[i])) {
         // a boundary particle with no fluid in the cells it walks has an empty list
         int cx, cy, cz;
         cell_of_key(k.gx, k.gy, keys[i], cx, cy, cz);
-        bool any = false;
-        const int r = k.reach;
-        for (int z = max(cz - r, 0); z <= min(cz + r, k.gz - 1); z++)
-            for (int y = max(cy - r, 0); y <= min(cy + r, k.gy - 1); y++) {
-                const int row = (z * k.gy + y) * k.gx;
-                for (int x = max(cx - r, 0); x <= min(cx + r, k.gx - 1); x++)
-                    any = any || __ldg(nl.fluid_cells + row + x) != 0;
-            }
-        if (!any) {
+        if (!near_fluid(k, cs, nl.rank, cx, cy, cz)) {
             nl.count[t] = 0;
             return;
         }

@@ -50,20 +50,6 @@ __device__ __forceinline__ size_t twin_col(const NbrList& nl, int u) {
 constexpr int TWIN_WALKS = -1;  // count of a thread one of whose particles overflowed its list
 
 // ---------------------------------------------------------------- list build
-template <class KP>
-__device__ __forceinline__ bool near_fluid(const KP& k, const unsigned char* __restrict__ fluid,
-                                           int cx, int cy, int cz) {
-    const int r = k.reach;
-    bool any = false;
-    for (int z = max(cz - r, 0); z <= min(cz + r, k.gz - 1); z++)
-        for (int y = max(cy - r, 0); y <= min(cy + r, k.gy - 1); y++) {
-            const int row = (z * k.gy + y) * k.gx;
-            for (int x = max(cx - r, 0); x <= min(cx + r, k.gx - 1); x++)
-                any = any || __ldg(fluid + row + x) != 0;
-        }
-    return any;
-}
-
 // One particle's side of the build: its cell and the part of a strip its cutoff sphere reaches.
 struct TwinWalk {
     int cx, cy, cz;
@@ -132,7 +118,7 @@ struct RingWriter {
 // The shared lists.  Bound by instructions (62% issue, 40% of the ALU pipe; about 390 candidates a
 // warp for 100 listed slots).  4.96M particles, 1.60 ms with a window per particle and strip and a
 // branch per candidate; 1.27 with one walk over the rows and cells either sphere reaches; 1.16 with
-// branch-free candidates on top.
+// branch-free candidates on top; 1.05 with near_fluid on the fluid ranks.
 template <class P>
 __global__ void __launch_bounds__(TWIN_BUILD_THREADS)
 k_nbr_build_twin(KParamsT<float> k, const float4* __restrict__ X,
@@ -156,9 +142,8 @@ k_nbr_build_twin(KParamsT<float> k, const float4* __restrict__ X,
     }
     const bool alla = fluid_rec(pa.w), allb = fluid_rec(pb.w);
     const TwinWalk wa = twin_walk<P>(k, pa, keys[a], cut2), wb = twin_walk<P>(k, pb, keys[b], cut2);
-    if (!alla && !allb && nl.fluid_cells &&
-        !(wa.on && near_fluid(k, nl.fluid_cells, wa.cx, wa.cy, wa.cz)) &&
-        !(wb.on && near_fluid(k, nl.fluid_cells, wb.cx, wb.cy, wb.cz))) {
+    if (!alla && !allb && nl.rank && !(wa.on && near_fluid(k, cs, nl.rank, wa.cx, wa.cy, wa.cz)) &&
+        !(wb.on && near_fluid(k, cs, nl.rank, wb.cx, wb.cy, wb.cz))) {
         nl.count[u] = 0;
         return;
     }

@@ -29,11 +29,9 @@ int key_bits_for(int num_cells);
 
 // ---------------------------------------------------------------- cell list (lib/mesh.cu)
 // Dense cell starts: cell_start[c] = first sorted slot whose key >= c, for c in [0, C];
-// cell_start[C] = n.  Keys must be sorted and < C.  With `type` and `fluid_cells` (C + 4 bytes),
-// also marks the cells that hold a fluid particle.
+// cell_start[C] = n.  Keys must be sorted and < C.
 cudaError_t build_cell_starts(const unsigned* sorted_keys, int n, int num_cells,
-                              int* cell_start, cudaStream_t s, const unsigned* gate = nullptr,
-                              const int* type = nullptr, unsigned char* fluid_cells = nullptr);
+                              int* cell_start, cudaStream_t s, const unsigned* gate = nullptr);
 
 // ---------------------------------------------------------------- precision policies
 // The resident solver in three precisions sharing one code path:
@@ -169,10 +167,10 @@ struct NbrList {
     // squared list cutoff chosen on the device at each rebuild (adaptive skin); NULL: the
     // constant block's kh2_list
     const float* cut2 = nullptr;
-    // cells holding a fluid particle (marked with the cell starts); NULL: not known.  A
-    // boundary particle keeps fluid neighbours only, so one with no such cell among its 27
-    // has an empty list without walking them.
-    const unsigned char* fluid_cells = nullptr;
+    // fluid slots before each slot (n + 1 entries, launch_work_order); NULL: not known.  A boundary
+    // particle keeps fluid neighbours only, so one with no fluid in the cells it walks has an
+    // empty list without walking them.  Read by the build only.
+    const int* rank = nullptr;
     // per-instance decisions (KParams::inst_boxes): the instance words and the instance of
     // every slot; the build skips the particles of instances that keep their lists.  NULL:
     // every particle is rebuilt at cut2
@@ -245,8 +243,8 @@ cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet
 // with_tmp: also the predictor's saved state; dense: also dst.xyz.
 // The work order of the list kernels (NbrList::order) of a cell-sorted set on `grid`: its fluid
 // slots, then the others, each in slot order or (rows) with pairs of rows merged so that
-// consecutive positions hold particles one above the other.  Scratch: rank (n + 1 ints) and
-// tiles (one word per 4096 slots).
+// consecutive positions hold particles one above the other.  Also fills rank (n + 1 ints: the fluid
+// slots before each slot).  Scratch: tiles (one word per 4096 slots).
 cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int* type,
                               const unsigned* keys, const int* cs, int* rank, unsigned* tiles,
                               int* order, cudaStream_t s, const unsigned* gate);
@@ -343,7 +341,6 @@ struct sph_ctx {
     unsigned* hash_x = nullptr;      // next cell of every slot of x
     unsigned* keys_sorted = nullptr; // sorted cell keys of y
     int* perm = nullptr;             // y slot k came from x slot perm[k]
-    unsigned char* fluid_cells = nullptr;  // cells holding fluid, per list build
     sph::Pass1Out p1;                // pass-1 output
     sph::ParticleSetT<double> xd, yd;
     sph::Pass1OutT<double> p1d;

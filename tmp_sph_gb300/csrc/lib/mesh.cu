@@ -270,13 +270,11 @@ cudaError_t fill_u32(unsigned* p, unsigned value, long count, const unsigned* ga
 
 // ---------------------------------------------------------------- dense cell starts
 __global__ void k_cell_mark(const unsigned* __restrict__ keys, int n, int num_cells,
-                            int* __restrict__ cs, const unsigned* gate,
-                            const int* __restrict__ type, unsigned char* __restrict__ fluid) {
+                            int* __restrict__ cs, const unsigned* gate) {
     if (gated_off(gate)) return;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     unsigned key = keys[k];
-    if (fluid && key < (unsigned)num_cells && type[k] == SPH_TYPE_FLUID) fluid[key] = 1;
     // key num_cells starts the tail of slots outside every cell (park_inactive)
     if ((k == 0 || keys[k - 1] != key) && key <= (unsigned)num_cells) cs[key] = k;
 }
@@ -351,9 +349,8 @@ k_cell_fill(int* __restrict__ cs, int num_cells, const unsigned* __restrict__ ke
     }
 }
 
-// Dense cell starts and fluid marks of a fine grid in one kernel: a block finds the slots of its
-// CS_CELLS cells, marks their first slots and kinds in shared memory and writes the cells out, each
-// once.  The general path (clear, mark, fill) writes every cell twice and reads it once, and its
+// Dense cell starts of a fine grid in one kernel: a block finds the slots of its CS_CELLS cells,
+// marks their first slots in shared memory and writes the cells out, each once.  The general path (clear, mark, fill) writes every cell twice and reads it once, and its
 // one-thread searches took 22 dependent loads a block.  4.96M particles on 50M cells: 0.31 ms there,
 // 0.09 here.  A block walks all slots of its cells, so this is for grids with more cells than
 // particles; coarse cells hold tens of thousands of slots per CS_CELLS.
@@ -364,10 +361,8 @@ constexpr int CS_ROUNDS = CS_CELLS / CS_THREADS;
 
 __global__ void __launch_bounds__(CS_THREADS)
 k_cell_starts(const unsigned* __restrict__ keys, int n, int num_cells, int* __restrict__ cs,
-              const int* __restrict__ type, unsigned char* __restrict__ fluid,
               const unsigned* gate) {
     __shared__ int s_start[CS_CELLS];
-    __shared__ __align__(4) unsigned char s_fluid[CS_CELLS];
     __shared__ int s_range[2];
     __shared__ int s_wmin[CS_WARPS];
     if (gated_off(gate)) return;
@@ -379,7 +374,6 @@ k_cell_starts(const unsigned* __restrict__ keys, int n, int num_cells, int* __re
         if (lane == 0) s_range[warp] = at;
     }
     for (int c = tid; c < CS_CELLS; c += CS_THREADS) s_start[c] = NONE;
-    for (int c = tid; c < CS_CELLS / 4; c += CS_THREADS) reinterpret_cast<unsigned*>(s_fluid)[c] = 0u;
     __syncthreads();
     const int k0 = s_range[0], k1 = s_range[1];
     for (int k = k0 + tid; k < k1; k += CS_THREADS) {
@@ -387,7 +381,6 @@ k_cell_starts(const unsigned* __restrict__ keys, int n, int num_cells, int* __re
         const long c = (long)key - c0;  // in [0, CS_CELLS): sorted keys between the two bounds
         if ((unsigned long)c >= (unsigned long)CS_CELLS) continue;
         if (k == k0 || keys[k - 1] != key) s_start[c] = k;
-        if (fluid && type[k] == SPH_TYPE_FLUID) s_fluid[c] = 1;
     }
     __syncthreads();
     // an empty cell takes the start of the next cell that is not: suffix minima, each warp over its
@@ -414,10 +407,6 @@ k_cell_starts(const unsigned* __restrict__ keys, int n, int num_cells, int* __re
         if (c <= num_cells) cs[c] = v;
         carry = __shfl_sync(0xffffffffu, v, 0);
     }
-    if (fluid)
-        for (int c = tid; c < CS_CELLS / 4; c += CS_THREADS)
-            if (c0 + 4L * c < num_cells)
-                reinterpret_cast<unsigned*>(fluid + c0)[c] = reinterpret_cast<unsigned*>(s_fluid)[c];
 }
 
 // ---------------------------------------------------------------- drop-in kernels
@@ -973,26 +962,17 @@ cudaError_t radix_sort_pairs(const unsigned* keys_in, const int* vals_in, unsign
 }
 
 cudaError_t build_cell_starts(const unsigned* sorted_keys, int n, int num_cells, int* cs,
-                              cudaStream_t s, const unsigned* gate, const int* type,
-                              unsigned char* fluid_cells) {
+                              cudaStream_t s, const unsigned* gate) {
     if (num_cells >= n) {
         k_cell_starts<<<blocks_for((long)num_cells + 1, CS_CELLS), CS_THREADS, 0, s>>>(
-            sorted_keys, n, num_cells, cs, type, type ? fluid_cells : nullptr, gate);
+            sorted_keys, n, num_cells, cs, gate);
         return cudaGetLastError();
     }
     cudaError_t e = fill_u32(reinterpret_cast<unsigned*>(cs), 0x7f7f7f7fu, (long)num_cells + 1,
                              gate, s);
     if (e != cudaSuccess) return e;
-    if (fluid_cells && type) {
-        e = fill_u32(reinterpret_cast<unsigned*>(fluid_cells), 0u, ((long)num_cells + 4) / 4,
-                     gate, s);
-        if (e != cudaSuccess) return e;
-    } else {
-        fluid_cells = nullptr;
-    }
     if (n > 0)
-        k_cell_mark<<<blocks_for(n, 256), 256, 0, s>>>(sorted_keys, n, num_cells, cs, gate, type,
-                                                       fluid_cells);
+        k_cell_mark<<<blocks_for(n, 256), 256, 0, s>>>(sorted_keys, n, num_cells, cs, gate);
     k_cell_fill<<<blocks_for((long)num_cells + 1, FILL_CHUNK), FILL_THREADS, 0, s>>>(
         cs, num_cells, sorted_keys, n, gate);
     return cudaGetLastError();

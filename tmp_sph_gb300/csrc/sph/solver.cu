@@ -147,8 +147,6 @@ void release(sph_ctx* c) {
     free_state(c);
     cudaFree(c->hash_x); cudaFree(c->keys_sorted); cudaFree(c->perm);
     cudaFree(c->cell_start); cudaFree(c->sort_scratch); cudaFree(c->err);
-    cudaFree(c->fluid_cells);
-    c->fluid_cells = nullptr;
     cudaFree(c->nl.idx); cudaFree(c->nl.count); cudaFree(c->nl.xb);
     c->nl = NbrList{};
     cudaFree(c->rb);
@@ -220,7 +218,9 @@ bool per_instance(const sph_ctx* c) {
 
 // The neighbour list to use this half step, or NULL to walk the cells in every pass.
 const NbrList* list_for(sph_ctx* c) {
-    c->nl.fluid_cells = c->fluid_cells;
+    // the work order's ranks stay in the pass-1 scratch until pass 1 writes there
+    c->nl.rank = c->prec == SPH_PREC_FP64 ? reinterpret_cast<const int*>(c->p1d.self)
+                                          : reinterpret_cast<const int*>(c->p1.self);
     c->nl.order = c->perm;
     const bool pi = per_instance(c);
     c->nl.iw = pi ? c->iw : nullptr;
@@ -593,8 +593,7 @@ cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, HalfStep
     if ((e = launch_gather<P>(k, c->perm, y, x, tmp, 0, c->keys_sorted, s, gate)) != cudaSuccess)
         return e;
     if ((e = launch_gather<P>(k, nullptr, x, y, tmp, 1, nullptr, s, gate)) != cudaSuccess) return e;
-    if ((e = build_cell_starts(c->keys_sorted, c->n, c->Pi.num_cells, c->cell_start, s, gate,
-                               y.type, c->fluid_cells)) !=
+    if ((e = build_cell_starts(c->keys_sorted, c->n, c->Pi.num_cells, c->cell_start, s, gate)) !=
         cudaSuccess)
         return e;
     // the permutation just applied, the sort's scratch and the pass-1 records hold nothing now
@@ -783,7 +782,6 @@ extern "C" int sph_create(const sph_params* p, int capacity, sph_ctx** out) {
     if (e == cudaSuccess) e = dalloc(&c->perm, cap);
     c->cell_capacity = std::max(p->num_cells, c->Pi.num_cells);
     if (e == cudaSuccess) e = dalloc(&c->cell_start, (size_t)c->cell_capacity + 1);
-    if (e == cudaSuccess) e = cudaMalloc(&c->fluid_cells, (size_t)c->cell_capacity + 4);
     c->sort_scratch_bytes = sort_scratch_bytes(cap);
     if (e == cudaSuccess) e = cudaMalloc(&c->sort_scratch, c->sort_scratch_bytes);
     if (e == cudaSuccess) e = dalloc(&c->err, 1);
@@ -832,18 +830,13 @@ extern "C" int sph_destroy(sph_ctx* c) {
 static cudaError_t ensure_cells(sph_ctx* c, int cells) {
     if (cells <= c->cell_capacity) return cudaSuccess;
     int* cs = nullptr;
-    unsigned char* fc = nullptr;
-    cudaError_t e = dalloc(&cs, (size_t)cells + 1);
-    if (e == cudaSuccess) e = cudaMalloc(&fc, (size_t)cells + 4);
+    const cudaError_t e = dalloc(&cs, (size_t)cells + 1);
     if (e != cudaSuccess) {
-        cudaFree(cs);
         cudaGetLastError();
         return e;
     }
     cudaFree(c->cell_start);
-    cudaFree(c->fluid_cells);
     c->cell_start = cs;
-    c->fluid_cells = fc;
     c->cell_capacity = cells;
     return cudaSuccess;
 }
@@ -1467,7 +1460,7 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
     // the drop-in builds and uses its list within this call, with the constant cutoff
     NbrList dl = c->nl;
     dl.cut2 = nullptr;
-    dl.fluid_cells = nullptr;
+    dl.rank = nullptr;
     dl.order = nullptr;
     const NbrList* nl = list_for(c) ? &dl : nullptr;
     if (nl && launch_nbr_build<PrecF32>(k, c->x, c->keys_sorted, c->cell_start, *nl,
