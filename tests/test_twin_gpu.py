@@ -99,3 +99,33 @@ def test_twin_batch_equals_solo(sphlib, cuda):
     for b in range(4):
         for k in ("pos", "vel", "rho", "p"):
             assert np.array_equal(out[k][b * n:(b + 1) * n], ref[k]), (b, k)
+
+
+def test_drop_in_ns_twin_gives_the_bits_of_one_particle_per_thread(sphlib, cuda):
+    """sph_ns over the threshold: the shared lists give the rates, divergence and wall values of the
+    one-particle path (which also returns the wall sums)."""
+    import torch
+    from gpu_util import dev, host
+    from tmp_sph_gb300 import solver as S
+    st, p = state(0.0061, True)
+    n = len(st["rho"])
+    h, idx = (torch.empty(n, dtype=torch.int32, device=cuda) for _ in range(2))
+    S.calc_hash(p, dev(st["pos"], cuda), h, idx, n)
+    S.sort_particles(h, idx, n)
+    cs = torch.empty(p.num_cells, dtype=torch.int32, device=cuda)
+    ce = torch.empty(p.num_cells, dtype=torch.int32, device=cuda)
+    keys = ("pos", "vel", "rho", "p", "type")
+    out = []
+    with S.Solver(p, n) as sol:
+        for sums in (False, True):
+            q = {k: torch.empty_like(dev(st[k], cuda)) for k in keys}
+            S.reorder(p, *(dev(st[k], cuda) for k in keys), None, *(q[k] for k in keys), None, h,
+                      idx, cs, ce, n)
+            r = {k: torch.empty(m, device=cuda) for k, m in (("rd", n), ("vd", 3 * n), ("dv", n),
+                                                             ("rs", n), ("ws", n))}
+            sol.ns(q["pos"], q["vel"], q["rho"], q["p"], q["type"], r["rd"], r["vd"], cs, ce, n, h,
+                   r["dv"], r["rs"] if sums else None, r["ws"] if sums else None)
+            out.append({k: host(v) for k, v in (("rd", r["rd"]), ("vd", r["vd"]), ("dv", r["dv"]),
+                                                ("rho", q["rho"]), ("p", q["p"]))})
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k

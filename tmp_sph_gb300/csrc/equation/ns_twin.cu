@@ -424,8 +424,9 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
 template <class P, int MODE>
 __global__ void __maxnreg__(104)
 k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ keys,
-             const int* __restrict__ cs, NbrList nl, Pass1Out p1, ParticleSet out,
-             unsigned* __restrict__ out_hash, unsigned* err, unsigned* disp) {
+             const int* __restrict__ cs, NbrList nl, Pass1Out p1, float* __restrict__ rho_dt,
+             float* __restrict__ vel_dt, ParticleSet out, unsigned* __restrict__ out_hash,
+             unsigned* err, unsigned* disp) {
     DispBox box;
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (2 * u < k.n) {
@@ -459,11 +460,11 @@ k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
 #pragma unroll 1
         for (int m = 0; m < (tw.two ? 2 : 1); m++) {
             const Pass2Acc<P, MODE> C = m ? B : A;
-            pass2_finish<P, MODE>(k, m ? tw.b : tw.a, C, in, keys, nl, nullptr, nullptr, 0, out,
+            pass2_finish<P, MODE>(k, m ? tw.b : tw.a, C, in, keys, nl, rho_dt, vel_dt, 0, out,
                                   out_hash, err, box, disp);
         }
     }
-    if (disp == nullptr) return;
+    if (MODE == MODE_RATES || disp == nullptr) return;
     // the block's displacement box; blockDim is a multiple of 32, every thread gets here
     __shared__ unsigned s_box[6 * (NS_MAX_THREADS / 32)];
     reduce_disp_box(box, disp, s_box);
@@ -500,10 +501,19 @@ cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet
     if (k.n <= 0) return cudaSuccess;
     if (half == HALF_PREDICT)
         k_pass2_twin<P, MODE_PRED><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(
-            k, in, keys, cs, nl, p1, out, out_hash, err, disp);
+            k, in, keys, cs, nl, p1, nullptr, nullptr, out, out_hash, err, disp);
     else
         k_pass2_twin<P, MODE_CORR><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(
-            k, in, keys, cs, nl, p1, out, out_hash, err, disp);
+            k, in, keys, cs, nl, p1, nullptr, nullptr, out, out_hash, err, disp);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pass2_rates_twin(const KParams& k, const ParticleSet& in, const unsigned* keys,
+                                    const int* cs, const NbrList& nl, const Pass1Out& p1,
+                                    float* rho_dt, float* vel_dt, cudaStream_t s) {
+    if (k.n <= 0) return cudaSuccess;
+    k_pass2_twin<PrecF32, MODE_RATES><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(
+        k, in, keys, cs, nl, p1, rho_dt, vel_dt, ParticleSet{}, nullptr, nullptr, nullptr);
     return cudaGetLastError();
 }
 

@@ -237,6 +237,10 @@ cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet
                               const Pass1Out& p1, ParticleSet out, unsigned* out_hash,
                               unsigned* err, unsigned* disp, cudaStream_t s);
 
+cudaError_t launch_pass2_rates_twin(const KParams& k, const ParticleSet& in, const unsigned* keys,
+                                    const int* cs, const NbrList& nl, const Pass1Out& p1,
+                                    float* rho_dt, float* vel_dt, cudaStream_t s);
+
 // Resident-state glue (lib/mesh.cu), one instantiation per precision policy P.
 // perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
 // cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).

@@ -1463,6 +1463,27 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
     dl.rank = nullptr;
     dl.order = nullptr;
     const NbrList* nl = list_for(c) ? &dl : nullptr;
+    // two particles per thread as on the resident path, the boundary particles after the fluid
+    // (their order, the ranks it takes and its tile counts go where the resident lists, which this
+    // call replaces, keep theirs); rates of boundary rows and the wall sums take the other path
+    if (nl && n >= TWIN_MIN_PARTICLES && !c->opt_wall_rates && !rhop_sum && !w_sum) {
+        dl.order = c->perm;
+        dl.rank = reinterpret_cast<const int*>(c->p1.self);
+        k.threads = 64;
+        if (launch_work_order(n, c->P, 0, c->x.type, c->keys_sorted, c->cell_start,
+                              reinterpret_cast<int*>(c->p1.self),
+                              static_cast<unsigned*>(c->sort_scratch), c->perm, s,
+                              nullptr) != cudaSuccess ||
+            launch_nbr_build_twin<PrecF32>(k, c->x, c->keys_sorted, c->cell_start, dl, c->p1.nrec,
+                                           c->err, s, nullptr) != cudaSuccess ||
+            launch_pass1_twin<PrecF32>(k, c->x, c->keys_sorted, c->cell_start, dl, c->p1, s) !=
+                cudaSuccess ||
+            launch_pass2_rates_twin(k, c->x, c->keys_sorted, c->cell_start, dl, c->p1, rho_dt,
+                                    vel_dt, s) != cudaSuccess ||
+            launch_ns_writeback(k, s_type, c->p1.self, s_rho, s_p, dofv, s) != cudaSuccess)
+            return SPH_ERR_CUDA;
+        return force_rebuild(c, s) == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
+    }
     if (nl && launch_nbr_build<PrecF32>(k, c->x, c->keys_sorted, c->cell_start, *nl,
                                         c->p1.nrec, c->opt_wall_rates, c->err, s) != cudaSuccess)
         return SPH_ERR_CUDA;
