@@ -86,8 +86,8 @@ __device__ __forceinline__ void visit_fluid(const KParamsT<float>& k, const NbrL
         for (int c = 0; c < 4; c++) ld_rec(R, P::kCodes ? slot_index(e[c]) : e[c], a[c], v[c]);
 #pragma unroll
         for (int c = 0; c < 4; c += 2)
-            acc.fluid_two(k, a[c], v[c], P::kCodes ? slot_code(e[c]) : 0u, a[c + 1], v[c + 1],
-                          P::kCodes ? slot_code(e[c + 1]) : 0u);
+            acc.fluid_two(k, a[c], v[c], P::kCodes ? (unsigned)e[c] : 0u, a[c + 1], v[c + 1],
+                          P::kCodes ? (unsigned)e[c + 1] : 0u);
     });
 }
 
@@ -120,7 +120,7 @@ __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
                 V a, b;
                 ld_rec(R, j, a, b);
                 T dx, dy, dz;
-                rel_pos<P>(k, acc.pi, a, P::kCodes ? slot_code(e) : 0u, dx, dy, dz);
+                rel_pos<P>(k, acc.pi, a, P::kCodes ? (unsigned)e : 0u, dx, dy, dz);
                 const T r2 = dist2(dx, dy, dz);
                 if (inside(r2, k.kh2)) f(j, a, b, dx, dy, dz, r2, ld_vol(vol, j));
             };
@@ -191,8 +191,8 @@ __device__ __forceinline__ void nbr_build_one(const KParamsT<typename P::T>& k,
                 float fx, fy, fz;
                 code_steps(code, fx, fy, fz);
                 const float sx = fma_rn(-fx, k.reach_cell, pi.x);
-                const float sy = fma_rn(-fy, k.reach_cell, pi.y);
-                const float sz = fma_rn(-fz, k.reach_cell, pi.z);
+                const float sy = fma_rn(-0.25f * fy, k.reach_cell, pi.y);
+                const float sz = fma_rn(-0.0625f * fz, k.reach_cell, pi.z);
 #pragma unroll 4
                 for (int j = j0; j < j1; j++) {
                     const vec4_t<T> pj = ld_pos(X, (size_t)j);

@@ -90,7 +90,7 @@ __device__ __forceinline__ void visit_group(const KParamsT<typename P::T>& k,
             V a, b;
             ld_rec(R, j, a, b);
             T dx, dy, dz;
-            rel_pos<P>(k, pi, a, P::kCodes ? slot_code(e) : 0u, dx, dy, dz);
+            rel_pos<P>(k, pi, a, P::kCodes ? (unsigned)e : 0u, dx, dy, dz);
             const T r2 = dist2(dx, dy, dz);
             if (inside(r2, k.kh2)) f(j, a, b, dx, dy, dz, r2, ld_vol(vol, j));
         };

@@ -20,14 +20,13 @@ namespace {
 // are picked by the autotuner.  ppt > 1 runs the grid-stride instantiation (GS), which holds
 // its loop state in registers (pass 2: 64 instead of 48), so ppt = 1 has its own.
 constexpr int NS_MAX_THREADS = 256;
-// Mixed precision: a list slot is j | code << CODE_SHIFT (j < 2^26), code the neighbour's
-// anchor cell relative to i's (cell_code).
-constexpr int CODE_SHIFT = 26;
-constexpr unsigned IDX_MASK = (1u << CODE_SHIFT) - 1u;
-__device__ __forceinline__ int slot_index(int e) { return (int)((unsigned)e & IDX_MASK); }
-__device__ __forceinline__ unsigned slot_code(int e) { return (unsigned)e >> CODE_SHIFT; }
+// Mixed precision: a list slot is j << CODE_BITS | code (j < 2^26), code the neighbour's anchor cell
+// relative to i's (cell_code).  The code sits in the low bits, where one logic operation per axis
+// turns its field into a float (code_steps).
+constexpr int CODE_BITS = 6;
+__device__ __forceinline__ int slot_index(int e) { return (int)((unsigned)e >> CODE_BITS); }
 __device__ __forceinline__ int make_slot(int j, unsigned code) {
-    return (int)((unsigned)j | (code << CODE_SHIFT));
+    return (int)((unsigned)j << CODE_BITS | code);
 }
 // Padding slot of a list of n particles: record n, which the build puts far outside any support
 // radius (pad_record), so evaluating it adds nothing.
@@ -432,12 +431,13 @@ __device__ __forceinline__ void for_each_candidate(const KP& k, const int* __res
     });
 }
 
-// The anchor steps of a mixed-precision cell code as floats: each 2-bit field f as f - 1,
-// without an integer conversion (the float with bits 0x4B000000 | f is 2^23 + f).
+// The anchor steps of a mixed-precision cell code (the low bits of `code`; a whole list slot will
+// do) as floats, without an integer conversion: the float with bits 0x4B000000 | v is 2^23 + v.
+// Each 2-bit field f as f - 1 times its place: 1, 4 and 16 for x, y and z.
 __device__ __forceinline__ void code_steps(unsigned code, float& fx, float& fy, float& fz) {
     fx = __fsub_rn(__uint_as_float(0x4B000000u | (code & 3u)), 8388609.0f);
-    fy = __fsub_rn(__uint_as_float(0x4B000000u | ((code >> 2) & 3u)), 8388609.0f);
-    fz = __fsub_rn(__uint_as_float(0x4B000000u | (code >> 4)), 8388609.0f);
+    fy = __fsub_rn(__uint_as_float(0x4B000000u | (code & 12u)), 8388612.0f);
+    fz = __fsub_rn(__uint_as_float(0x4B000000u | (code & 48u)), 8388624.0f);
 }
 
 // One record (two vec4) in single 256-bit read-only loads: a neighbour gather touches one L1
@@ -519,6 +519,20 @@ __device__ __forceinline__ F2 fma2_rn(F2 a, F2 b, F2 c) {
     return r;
 }
 
+// A difference of offsets moved into i's anchor frame: d - (anchor steps of the code) * reach_cell,
+// one explicitly rounded fused multiply-add per axis, so every caller (list, cell walk) gets the same
+// bits.  The constants carry the fields' places (a power of two: the same products), x and y go in
+// two-lane instructions: seven instructions for the decode and shift of a slot.
+__device__ __forceinline__ void anchor_shift(const KParamsT<float>& k, unsigned code, float& dx,
+                                             float& dy, float& dz) {
+    const F2 f = add2_rn(pack2(__uint_as_float(0x4B000000u | (code & 3u)),
+                               __uint_as_float(0x4B000000u | (code & 12u))),
+                         F2{k.code_bias2});
+    unpack2(fma2_rn(f, F2{k.m_anchor2}, pack2(dx, dy)), dx, dy);
+    const float fz = __fsub_rn(__uint_as_float(0x4B000000u | (code & 48u)), 8388624.0f);
+    dz = fma_rn(fz, k.m_anchor_z, dz);
+}
+
 // Relative position r = x_i - x_j of a pair: from positions in the simulation's frame, or
 // (cell codes) from the offsets from their anchor cells and j's anchor relative to i's
 // (anchor steps of reach cells).
@@ -528,16 +542,9 @@ __device__ __forceinline__ void rel_pos(const KParamsT<typename P::T>& k, const 
                                         typename P::T& dy, typename P::T& dz) {
     using T = typename P::T;
     if constexpr (P::kCodes) {
-        // one explicitly rounded difference and one fused multiply-add per axis, so every
-        // caller (list, cell walk, list build) gets the same bits whatever the compiler hoists
-        // the anchor steps of the code times one anchor step reach * cell
-        float fx, fy, fz;
-        code_steps(code, fx, fy, fz);
-        float ox, oy;
-        sub2_rn(pi.x, pi.y, pj.x, pj.y, ox, oy);
-        dx = fma_rn(-fx, k.reach_cell, ox);
-        dy = fma_rn(-fy, k.reach_cell, oy);
-        dz = fma_rn(-fz, k.reach_cell, sub_rn(pi.z, pj.z));
+        sub2_rn(pi.x, pi.y, pj.x, pj.y, dx, dy);
+        dz = sub_rn(pi.z, pj.z);
+        anchor_shift(k, code, dx, dy, dz);
     } else {
         (void)k;
         (void)code;
@@ -554,13 +561,7 @@ __device__ __forceinline__ void rel_pos_s(const KParamsT<float>& k, const float4
                                           float& dz, float& s) {
     sub2_rn(pi.x, pi.y, pj.x, pj.y, dx, dy);
     sub2_rn(pi.z, s0, pj.z, pj.w, dz, s);
-    if constexpr (P::kCodes) {
-        float fx, fy, fz;
-        code_steps(code, fx, fy, fz);
-        dx = fma_rn(-fx, k.reach_cell, dx);
-        dy = fma_rn(-fy, k.reach_cell, dy);
-        dz = fma_rn(-fz, k.reach_cell, dz);
-    }
+    if constexpr (P::kCodes) anchor_shift(k, code, dx, dy, dz);
 }
 
 // Walk the cells of particle i over the positions X[STRIDE * j] and call

@@ -87,6 +87,10 @@ struct KParamsT {
     // 1: batched instances keep a displacement box each and rebuild their lists on their own
     // decisions (IW_* words below); 0: one box and one decision for all particles
     int inst_boxes;
+    // mixed precision: minus one anchor step over the places 1, 4 and 16 of a cell code's fields
+    // (x and y in m_anchor2), and the bias of the x and y fields as floats
+    unsigned long long m_anchor2, code_bias2;
+    T m_anchor_z;
     // FP32 constants of the pair arithmetic twice over, as operands of two-lane instructions
     // (unused by the FP64 kernels)
     unsigned long long inv_h2, m_half_inv_h2, one2, m_half2, c_fr2, c_fr_mass2, eta2_2,
@@ -95,6 +99,8 @@ struct KParamsT {
 using KParams = KParamsT<float>;
 
 KParams make_kparams(const sph_params& p, int n);
+// Two FP32 values as the operand of a two-lane instruction.
+unsigned long long two_floats(float lo, float hi);
 template <class T> KParamsT<T> make_kparams_t(const sph_params& p, int n);
 
 // ---------------------------------------------------------------- cell math

@@ -106,7 +106,7 @@ template <class T>
 __device__ __forceinline__ T pair_volume(const KParamsT<T>& k, T rho) {
     return k.c_fr_mass / rho;
 }
-// The list slots carry a cell code above a 26-bit neighbour index.
+// The list slots carry a cell code below a 26-bit neighbour index.
 inline bool prec_has_codes(int prec) {
     return prec == SPH_PREC_MIXED || prec == SPH_PREC_MIXED_COMP;
 }
@@ -156,9 +156,9 @@ enum HalfStep { HALF_PREDICT = 0, HALF_CORRECT = 1 };
 // the position i had when the list was built (its record position).  The list
 // holds every pair closer than the list cutoff (KParams::kh2_list, the support radius plus a
 // skin), in candidate-walk order; count[i] > cap means the list overflowed for i and the
-// passes walk the cells for it instead.  With cell codes (kCodes) each slot also holds, in
-// bits 26-31, the neighbour's anchor relative to i's ((dz+1) << 4 | (dy+1) << 2 | (dx+1)),
-// from which the passes rebuild relative positions out of the cell-local offsets.
+// passes walk the cells for it instead.  With cell codes (kCodes) a slot holds the index above six
+// bits with the neighbour's anchor relative to i's ((dz+1) << 4 | (dy+1) << 2 | (dx+1)), from
+// which the passes rebuild relative positions out of the cell-local offsets.
 struct NbrList {
     int* idx = nullptr;
     int* count = nullptr;

@@ -11,13 +11,6 @@ namespace {
 
 constexpr double kPi = 3.141592654;  // the reference's PI (src/header/sph.cuh:4)
 
-// An FP32 value in both halves of a two-lane operand.
-unsigned long long twice(float v) {
-    unsigned u;
-    std::memcpy(&u, &v, sizeof(u));
-    return (unsigned long long)u << 32 | u;
-}
-
 void fill_grid(sph_params* P, double pad, const float dmin[3], const float dmax[3]) {
     for (int c = 0; c < 3; c++) {
         P->grid_min[c] = (float)((double)dmin[c] - pad);
@@ -31,6 +24,14 @@ void fill_grid(sph_params* P, double pad, const float dmin[3], const float dmax[
 }  // namespace
 
 namespace sph {
+
+unsigned long long two_floats(float lo, float hi) {
+    unsigned u, v;
+    std::memcpy(&u, &lo, sizeof(u));
+    std::memcpy(&v, &hi, sizeof(v));
+    return (unsigned long long)v << 32 | u;
+}
+static unsigned long long twice(float v) { return two_floats(v, v); }
 
 KParams make_kparams(const sph_params& p, int n) {
     KParams k{};
@@ -88,6 +89,7 @@ KParams make_kparams(const sph_params& p, int n) {
     k.park_z = p.escape_park[2];
     k.park_inactive = p.park_inactive;
     k.inst_boxes = 0;
+    k.code_bias2 = two_floats(-8388609.f, -8388612.f);
     k.inv_h2 = twice(k.inv_h);
     k.m_half_inv_h2 = twice(-0.5f * k.inv_h);
     k.one2 = twice(1.f);

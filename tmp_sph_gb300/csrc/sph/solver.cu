@@ -343,6 +343,8 @@ KParamsT<T> resident_kparams(const sph_ctx* c) {
     k.list_win = k.lanes > 1;
     k.reach = c->opt_reach;
     k.reach_cell = (T)c->opt_reach * k.cell;
+    k.m_anchor2 = two_floats(-(float)k.reach_cell, -0.25f * (float)k.reach_cell);
+    k.m_anchor_z = (T)-0.0625 * k.reach_cell;
     k.gz_stride = c->n_inst > 1 ? instance_stride(c->gz_inst, c->opt_reach) : c->gz_inst;
     k.inst_boxes = per_instance(c) ? 1 : 0;
     k.inst_cells = c->n_inst > 1 ? c->Pi.grid_dim[0] * c->Pi.grid_dim[1] * k.gz_stride : 0;
