@@ -73,29 +73,68 @@ enum { LIST_NONE = 0, LIST_PLAIN = 1, LIST_WIN = 2 };
 template <class P>
 constexpr bool kPairTwo = std::is_same<typename P::T, float>::value && !P::kComp;
 
+// The records of a chunk's four slots, and the pairs of a fluid particle with them in list order.
+template <class P>
+__device__ __forceinline__ void load_chunk(const float4* __restrict__ R, const int4& q,
+                                           float4 (&a)[4], float4 (&v)[4]) {
+    const int e[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int c = 0; c < 4; c++) ld_rec(R, P::kCodes ? slot_index(e[c]) : e[c], a[c], v[c]);
+}
+template <class P, class Acc>
+__device__ __forceinline__ void pair_chunk(const KParamsT<float>& k, const int4& q,
+                                           const float4 (&a)[4], const float4 (&v)[4], Acc& acc) {
+    const int e[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int c = 0; c < 4; c += 2)
+        acc.fluid_two(k, a[c], v[c], P::kCodes ? (unsigned)e[c] : 0u, a[c + 1], v[c + 1],
+                      P::kCodes ? (unsigned)e[c + 1] : 0u);
+}
+
 // Listed neighbours of a fluid particle, a chunk of four at a time: the four record gathers are
-// issued together and the pairs evaluated without a branch, in list order.
-template <class P, bool WIN, class Acc>
+// issued together and the pairs evaluated without a branch, in list order.  DEEP: the records of the
+// next chunk are in flight while the current one is evaluated (twice the registers), for runs too
+// small to fill the SMs with warps, where the latency of a gather is all there is to hide.
+template <class P, bool WIN, bool DEEP, class Acc>
 __device__ __forceinline__ void visit_fluid(const KParamsT<float>& k, const NbrList& nl,
                                             const float4* __restrict__ R, int t, int cnt,
                                             Acc& acc) {
-    for_each_chunk<WIN>(nl.idx + nbr_col(nl, t), cnt, 0, 1, [&](const int4& q) {
-        const int e[4] = {q.x, q.y, q.z, q.w};
-        float4 a[4], v[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) ld_rec(R, P::kCodes ? slot_index(e[c]) : e[c], a[c], v[c]);
-#pragma unroll
-        for (int c = 0; c < 4; c += 2)
-            acc.fluid_two(k, a[c], v[c], P::kCodes ? (unsigned)e[c] : 0u, a[c + 1], v[c + 1],
-                          P::kCodes ? (unsigned)e[c + 1] : 0u);
-    });
+    const int* __restrict__ col = nl.idx + nbr_col(nl, t);
+    if constexpr (DEEP) {
+        const int pad = pad_slot<P>(k.n);
+        auto slots = [&](int c) {
+            return chunk_first<WIN>(c) < cnt ? ld_slots(col + ((size_t)c << 7))
+                                             : make_int4(pad, pad, pad, pad);
+        };
+        if (cnt <= 0) return;
+        int4 q0 = slots(0), q1 = slots(1), q2 = slots(2);
+        float4 a0[4], v0[4], a1[4], v1[4];
+        load_chunk<P>(R, q0, a0, v0);
+#pragma unroll 1
+        for (int c = 0; chunk_first<WIN>(c) < cnt; c += 2) {
+            load_chunk<P>(R, q1, a1, v1);
+            const int4 q3 = slots(c + 3);
+            pair_chunk<P>(k, q0, a0, v0, acc);
+            q0 = q2;
+            load_chunk<P>(R, q0, a0, v0);
+            q2 = slots(c + 4);
+            pair_chunk<P>(k, q1, a1, v1, acc);
+            q1 = q3;
+        }
+    } else {
+        for_each_chunk<WIN>(col, cnt, 0, 1, [&](const int4& q) {
+            float4 a[4], v[4];
+            load_chunk<P>(R, q, a, v);
+            pair_chunk<P>(k, q, a, v, acc);
+        });
+    }
 }
 
-// Neighbours of slot i (work position t; r2 < kh2) with their records R[2j], R[2j+1]: from the list (pairs in the skin
-// beyond the support radius are skipped), or by walking the cells over X[XSTRIDE * j] when i
-// overflowed the list.  f(j, a, b, dx, dy, dz, r2, vol); with FAST and kPairTwo the list goes through
-// acc.fluid_two instead (a fluid particle).
-template <class P, int LIST, int XSTRIDE, class Acc, class F>
+// Neighbours of slot i (work position t; r2 < kh2) with their records R[2j], R[2j+1]: from the list
+// (pairs in the skin beyond the support radius are skipped), or by walking the cells over
+// X[XSTRIDE * j] when i overflowed the list.  f(j, a, b, dx, dy, dz, r2, vol); with kPairTwo the list
+// of a fluid particle goes through acc.fluid_two instead.
+template <class P, int LIST, int XSTRIDE, bool DEEP, class Acc, class F>
 __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
                                               const int* __restrict__ cs,
                                               const unsigned* __restrict__ keys,
@@ -111,7 +150,7 @@ __device__ __forceinline__ void visit_records(const KParamsT<typename P::T>& k,
         if (cnt <= nl.cap) {
             if constexpr (kPairTwo<P>) {
                 if (acc.fi) {
-                    visit_fluid<P, LIST == LIST_WIN>(k, nl, R, t, cnt, acc);
+                    visit_fluid<P, LIST == LIST_WIN, DEEP>(k, nl, R, t, cnt, acc);
                     return;
                 }
             }
@@ -249,7 +288,7 @@ k_nbr_build(KParamsT<typename P::T> k, const vec4_t<typename P::T>* __restrict__
     }
 }
 
-template <class P, bool WRITE_SUMS, int LIST>
+template <class P, bool WRITE_SUMS, int LIST, bool DEEP>
 __device__ __forceinline__ void pass1_one(const KParamsT<typename P::T>& k,
                                           const ParticleSetT<typename P::T>& in,
                                           const unsigned* __restrict__ keys,
@@ -264,7 +303,7 @@ __device__ __forceinline__ void pass1_one(const KParamsT<typename P::T>& k,
     acc.load(in.rec, i);
     // a particle whose list overflowed walks the records' positions, a pass without lists the dense
     // ones of this half step's rebuild
-    visit_records<P, LIST, LIST == LIST_NONE ? 1 : 2>(k, cs, keys, nl,
+    visit_records<P, LIST, LIST == LIST_NONE ? 1 : 2, DEEP>(k, cs, keys, nl,
                               LIST == LIST_NONE ? in.xyz : in.rec, in.rec, in.vol, t, i, acc,
                               [&](int, const V& aj, const V& vj, T dx, T dy, T dz, T r2, T vol) {
         acc.pair(k, aj, vj, dx, dy, dz, r2, vol);
@@ -272,24 +311,24 @@ __device__ __forceinline__ void pass1_one(const KParamsT<typename P::T>& k,
     acc.template finish<WRITE_SUMS>(k, out, rhop_sum, w_sum, i);
 }
 
-// Registers of pass 1: room for the four records of a chunk in flight.
-template <class P>
-constexpr int kPass1Regs = std::is_same<typename P::T, double>::value ? 96 : 72;
+// Registers of pass 1: room for the four records of a chunk in flight, or (DEEP) two chunks.
+template <class P, bool DEEP>
+constexpr int kPass1Regs = DEEP ? 144 : std::is_same<typename P::T, double>::value ? 96 : 72;
 
-template <class P, bool WRITE_SUMS, int LIST, bool GS>
-__global__ void __maxnreg__(kPass1Regs<P>)
+template <class P, bool WRITE_SUMS, int LIST, bool GS, bool DEEP = false>
+__global__ void __maxnreg__((kPass1Regs<P, DEEP>))
 k_pass1(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         const unsigned* __restrict__ keys, const int* __restrict__ cs, NbrList nl,
         Pass1OutT<typename P::T> out, float* __restrict__ rhop_sum, float* __restrict__ w_sum) {
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (GS) {
         for (int i = i0; i < k.n; i += gridDim.x * blockDim.x)
-            pass1_one<P, WRITE_SUMS, LIST>(k, in, keys, cs, nl, out, rhop_sum, w_sum, i);
+            pass1_one<P, WRITE_SUMS, LIST, DEEP>(k, in, keys, cs, nl, out, rhop_sum, w_sum, i);
     } else if (i0 < k.n) {
-        pass1_one<P, WRITE_SUMS, LIST>(k, in, keys, cs, nl, out, rhop_sum, w_sum, i0);
+        pass1_one<P, WRITE_SUMS, LIST, DEEP>(k, in, keys, cs, nl, out, rhop_sum, w_sum, i0);
     }
 }
-template <class P, int MODE, int LIST>
+template <class P, int MODE, int LIST, bool DEEP>
 __device__ __forceinline__ void pass2_one(const KParamsT<typename P::T>& k, int t,
                                           const ParticleSetT<typename P::T>& in,
                                           const unsigned* __restrict__ keys,
@@ -305,7 +344,7 @@ __device__ __forceinline__ void pass2_one(const KParamsT<typename P::T>& k, int 
     Pass2Acc<P, MODE> acc;
     acc.load(k, p1, i, wall_rates);
     if (acc.active)
-        visit_records<P, LIST, 2>(k, cs, keys, nl, p1.nrec, p1.nrec, p1.vol, t, i, acc,
+        visit_records<P, LIST, 2, DEEP>(k, cs, keys, nl, p1.nrec, p1.nrec, p1.vol, t, i, acc,
                                   [&](int j, const V& aj, const V& vj, T dx, T dy, T dz, T r2,
                                       T vol) {
             acc.pair(k, p1, j, aj, vj, dx, dy, dz, r2, vol);
@@ -326,10 +365,10 @@ k_pass2(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (GS) {
         for (int i = i0; i < k.n; i += gridDim.x * blockDim.x)
-            pass2_one<P, MODE, LIST>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
+            pass2_one<P, MODE, LIST, false>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
                                      out_hash, err, box, disp);
     } else if (i0 < k.n) {
-        pass2_one<P, MODE, LIST>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
+        pass2_one<P, MODE, LIST, false>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
                                  out_hash, err, box, disp);
     }
     if (MODE == MODE_RATES || disp == nullptr) return;
@@ -342,7 +381,7 @@ k_pass2(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
 // The same kernel held to CAP registers (one particle per thread): room for a chunk's four records
 // in flight with the most warps that leaves.  At 133,968 particles (linear EOS) 80 registers run
 // in 29 us, 64 in 35, 48 in 49, against 44 for one gather at a time in 40; at 380,000 80 run in
-// 45 us, 96 in 55.  The kernel on cell-local offsets keeps 72 (380,000 particles: 77 us, 79 at 80,
+// 45 us, 96 in 55.  More than 100 registers: the deep form (visit_fluid).  The kernel on cell-local offsets keeps 72 (380,000 particles: 77 us, 79 at 80,
 // 83 at 64).
 template <class P, int MODE, int LIST, bool GS, int CAP>
 __global__ void __maxnreg__(CAP)
@@ -355,10 +394,10 @@ k_pass2_cap(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (GS) {
         for (int i = i0; i < k.n; i += gridDim.x * blockDim.x)
-            pass2_one<P, MODE, LIST>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
+            pass2_one<P, MODE, LIST, (CAP > 100)>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
                                      out_hash, err, box, disp);
     } else if (i0 < k.n) {
-        pass2_one<P, MODE, LIST>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
+        pass2_one<P, MODE, LIST, (CAP > 100)>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
                                  out_hash, err, box, disp);
     }
     if (MODE == MODE_RATES || disp == nullptr) return;
@@ -394,11 +433,23 @@ void pass1_launch_gs(const KParamsT<typename P::T>& k, const ParticleSetT<typena
                                                         nullptr);
 }
 
+// Below this many particles the passes run their deep form.  27,288 particles, five steps: FP32 292
+// us against 328, cell-local offsets 318 against 380; at 133,968 it has too few warps left (ten
+// steps 1.20 ms against 1.11).
+constexpr int DEEP_MAX_PARTICLES = 60000;
+
 template <class P, int LIST>
 void pass1_launch(const KParamsT<typename P::T>& k, const ParticleSetT<typename P::T>& in,
                   const unsigned* keys, const int* cs, const NbrList& nl,
                   const Pass1OutT<typename P::T>& o, float* rhop_sum, float* w_sum,
                   cudaStream_t s) {
+    if constexpr (LIST == LIST_PLAIN && kPairTwo<P>) {
+        if (k.ppt <= 1 && k.n < DEEP_MAX_PARTICLES && !rhop_sum && !w_sum) {
+            k_pass1<P, false, LIST, false, true><<<ns_grid(k), k.threads, 0, s>>>(
+                k, in, keys, cs, nl, o, nullptr, nullptr);
+            return;
+        }
+    }
     if (k.ppt > 1)
         pass1_launch_gs<P, LIST, true>(k, in, keys, cs, nl, o, rhop_sum, w_sum, s);
     else
@@ -421,6 +472,14 @@ void pass2_launch_gs(const KParamsT<typename P::T>& k, const ParticleSetT<typena
     auto with_list = [&](auto mode) {
         constexpr int L = decltype(mode)::value;
         if constexpr (MODE != MODE_RATES && !GS && (P::kId == SPH_PREC_FP32 || P::kMixed)) {
+            if constexpr (L == LIST_PLAIN && kPairTwo<P>) {
+                if (k.n < DEEP_MAX_PARTICLES) {
+                    k_pass2_cap<P, MODE, L, GS, 168><<<b, k.threads, 0, s>>>(
+                        k, in, keys, cs, *nl, p1, rho_dt, vel_dt, wall_rates, out, out_hash, err,
+                        disp);
+                    return;
+                }
+            }
             constexpr int cap = P::kCodes ? 72 : 80;
             k_pass2_cap<P, MODE, L, GS, cap><<<b, k.threads, 0, s>>>(
                 k, in, keys, cs, *nl, p1, rho_dt, vel_dt, wall_rates, out, out_hash, err, disp);
