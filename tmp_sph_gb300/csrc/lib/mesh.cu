@@ -36,6 +36,7 @@ struct SortScratch {
     int* vals_alt;
     unsigned* hist;    // [RS_RADIX][tiles]
     unsigned* totals;  // [RS_MAX_PASSES][RS_RADIX]
+    unsigned* spread;  // OR of all keys, OR of their complements
 };
 
 SortScratch carve(void* base, int n) {
@@ -49,6 +50,7 @@ SortScratch carve(void* base, int n) {
     s.hist = reinterpret_cast<unsigned*>(p);
     p += align256((size_t)RS_RADIX * (size_t)(rs_tiles(n) > 0 ? rs_tiles(n) : 1) * sizeof(unsigned));
     s.totals = reinterpret_cast<unsigned*>(p);
+    s.spread = s.totals + RS_MAX_PASSES * RS_RADIX;
     return s;
 }
 
@@ -74,8 +76,6 @@ __device__ __forceinline__ unsigned digit_peers(unsigned d, bool valid) {
     return peers;
 }
 
-// Per-tile digit histogram: hist[d * tiles + tile]; totals[d] accumulates over tiles.
-__global__ void __launch_bounds__(RS_THREADS)
 // Whether every key has the same digit at `shift` (a bit on which two keys differ is set in the OR
 // of the keys and in the OR of their complements): that pass moves nothing, and its kernels copy.
 // A 32-bit sort of cell keys below 2^24 has such a pass: its upsweep, scan and downsweep take 36 us
@@ -84,21 +84,29 @@ __device__ __forceinline__ bool same_digit(const unsigned* __restrict__ spread, 
     return ((spread[0] & spread[1]) >> shift & 0xffu) == 0u;
 }
 
+// Per-tile digit histogram: hist[d * tiles + tile]; totals[d] accumulates over tiles.
+__global__ void __launch_bounds__(RS_THREADS)
 k_rs_upsweep(const unsigned* __restrict__ keys, int n, int shift, unsigned xmask,
              int check_bits, unsigned* __restrict__ hist, int tiles,
-             unsigned* __restrict__ totals, unsigned* err, const unsigned* gate) {
+             unsigned* __restrict__ totals, unsigned* __restrict__ spread, unsigned* err,
+             const unsigned* gate) {
     __shared__ unsigned cnt[RS_RADIX];
     if (gated_off(gate)) return;
+    if (shift > 0 && same_digit(spread, shift)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < RS_RADIX) cnt[tid] = 0;
     __syncthreads();
     const long base = (long)blockIdx.x * RS_TILE + warp * (32 * RS_IPT) + lane;
-    unsigned flags = 0;
+    unsigned flags = 0, ones = 0, zeros = 0;
 #pragma unroll
     for (int r = 0; r < RS_IPT; r++) {
         long idx = base + r * 32;
         bool valid = idx < n;
         unsigned key = valid ? (__ldg(keys + idx) ^ xmask) : 0u;
+        if (valid) {
+            ones |= key;
+            zeros |= ~key;
+        }
         if (valid && check_bits < 32 && (key >> check_bits) != 0u) flags |= SPH_FLAG_KEY_RANGE;
         unsigned d = (key >> shift) & 0xffu;
         unsigned peers = digit_peers(d, valid);
@@ -110,6 +118,13 @@ k_rs_upsweep(const unsigned* __restrict__ keys, int n, int shift, unsigned xmask
         hist[(size_t)tid * tiles + blockIdx.x] = c;
         if (c) atomicAdd(&totals[tid], c);
     }
+    if (shift == 0) {  // the first pass sees every key: the spread for the later ones
+        ones = __reduce_or_sync(0xffffffffu, ones);
+        zeros = __reduce_or_sync(0xffffffffu, zeros);
+        // few blocks change the words once the first have written them
+        if (lane == 0 && (ones & ~*(volatile unsigned*)spread)) atomicOr(spread, ones);
+        if (lane == 0 && (zeros & ~*(volatile unsigned*)(spread + 1))) atomicOr(spread + 1, zeros);
+    }
     raise_flags(err, flags);
 }
 
@@ -118,11 +133,12 @@ constexpr int SC_THREADS = 256;
 // Exclusive scan of one digit's row of tile counts, offset by the counts of all smaller
 // digits: after this, hist[d * tiles + t] is the first output slot of digit d in tile t.
 __global__ void __launch_bounds__(SC_THREADS)
-k_rs_scan(unsigned* __restrict__ hist, int tiles, const unsigned* __restrict__ totals,
-          const unsigned* gate) {
+k_rs_scan(unsigned* __restrict__ hist, int tiles, const unsigned* __restrict__ totals, int shift,
+          const unsigned* __restrict__ spread, const unsigned* gate) {
     __shared__ unsigned wsum[(SC_THREADS / 32)];
     __shared__ unsigned s_carry;
     if (gated_off(gate)) return;
+    if (shift > 0 && same_digit(spread, shift)) return;
     const int d = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // base = sum of totals of digits < d
     unsigned v = (tid < d) ? totals[tid] : 0u;
@@ -168,7 +184,8 @@ __global__ void __launch_bounds__(RS_THREADS)
 k_rs_downsweep(const unsigned* __restrict__ keys_in, const int* __restrict__ vals_in,
                unsigned* __restrict__ keys_out, int* __restrict__ vals_out,
                const unsigned* __restrict__ hist, int n, int shift, unsigned xmask_in,
-               unsigned xmask_out, int tiles, const unsigned* gate) {
+               unsigned xmask_out, int tiles, const unsigned* __restrict__ spread,
+               const unsigned* gate) {
     __shared__ unsigned short s_cnt[RS_WARPS][RS_RADIX];  // a tile holds 4096 keys
     __shared__ unsigned s_gbase[RS_RADIX];
     __shared__ unsigned s_tpre[RS_RADIX];
@@ -178,6 +195,16 @@ k_rs_downsweep(const unsigned* __restrict__ keys_in, const int* __restrict__ val
 
     if (gated_off(gate)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (shift > 0 && same_digit(spread, shift)) {
+        for (int r = 0; r < RS_IPT; r++) {
+            const long idx = (long)blockIdx.x * RS_TILE + r * RS_THREADS + tid;
+            if (idx < n) {
+                keys_out[idx] = __ldg(keys_in + idx) ^ xmask_in ^ xmask_out;
+                vals_out[idx] = vals_in ? __ldg(vals_in + idx) : (int)idx;
+            }
+        }
+        return;
+    }
     if (tid < RS_RADIX)
 #pragma unroll
         for (int w = 0; w < RS_WARPS; w++) s_cnt[w][tid] = 0;
@@ -907,7 +934,7 @@ size_t sort_scratch_bytes(int n) {
     size_t tiles = (size_t)(rs_tiles(n) > 0 ? rs_tiles(n) : 1);
     return align256(nn * sizeof(unsigned)) + align256(nn * sizeof(int)) +
            align256((size_t)RS_RADIX * tiles * sizeof(unsigned)) +
-           align256((size_t)RS_MAX_PASSES * RS_RADIX * sizeof(unsigned));
+           align256(((size_t)RS_MAX_PASSES * RS_RADIX + 2) * sizeof(unsigned));
 }
 
 cudaError_t radix_sort_pairs(const unsigned* keys_in, const int* vals_in, unsigned* keys_out,
@@ -924,7 +951,7 @@ cudaError_t radix_sort_pairs(const unsigned* keys_in, const int* vals_in, unsign
     SortScratch sc = carve(scratch, n);
     const int tiles = rs_tiles(n);
     const unsigned xm = key_bits == 32 ? 0x80000000u : 0u;  // signed order for full keys
-    cudaError_t e = fill_u32(sc.totals, 0u, (long)RS_MAX_PASSES * RS_RADIX, gate, s);
+    cudaError_t e = fill_u32(sc.totals, 0u, (long)RS_MAX_PASSES * RS_RADIX + 2, gate, s);
     if (e != cudaSuccess) return e;
     const unsigned* kin = keys_in;
     const int* vin = vals_in;
@@ -953,10 +980,10 @@ cudaError_t radix_sort_pairs(const unsigned* keys_in, const int* vals_in, unsign
         const unsigned xout = (p == passes - 1) ? xm : 0u;
         unsigned* totals = sc.totals + (size_t)p * RS_RADIX;
         k_rs_upsweep<<<tiles, RS_THREADS, 0, s>>>(kin, n, shift, xin, p == 0 ? key_bits : 32,
-                                                   sc.hist, tiles, totals, err, gate);
-        k_rs_scan<<<RS_RADIX, SC_THREADS, 0, s>>>(sc.hist, tiles, totals, gate);
+                                                   sc.hist, tiles, totals, sc.spread, err, gate);
+        k_rs_scan<<<RS_RADIX, SC_THREADS, 0, s>>>(sc.hist, tiles, totals, shift, sc.spread, gate);
         k_rs_downsweep<<<tiles, RS_THREADS, 0, s>>>(kin, vin, kdst, vdst, sc.hist, n, shift, xin,
-                                                     xout, tiles, gate);
+                                                     xout, tiles, sc.spread, gate);
         kin = kdst;
         vin = vdst;
     }
