@@ -62,7 +62,7 @@ B_HASH, B_SORT, B_PERMUTE, B_PASS1, B_PASS2, B_INTEGRATE = 20, 16, 80, 52, 60, 1
 PHASE_BYTES = {"sort": B_SORT, "gather_cells": B_PERMUTE, "nbr_build": 16, "pass1": B_PASS1,
                "pass2_integrate": B_PASS2 + B_INTEGRATE + B_HASH}
 PHASE_KERNEL = {"sort": "k_rs_upsweep/k_rs_scan/k_rs_downsweep",
-                "gather_cells": "k_gather + k_cell_mark/k_cell_fill",
+                "gather_cells": "k_gather + k_cell_starts (k_cell_mark/k_cell_fill) + k_work_order",
                 "nbr_build": "k_nbr_build (one cell walk; positions read once = 16 B)",
                 "pass1": "k_pass1 (k_pass1_g with two or four lanes)",
                 "pass2_integrate": "k_pass2<MODE_PRED|MODE_CORR>"}
@@ -183,9 +183,10 @@ def build_case(name: str):
 
 
 def count_launches(num_cells: int, half_steps: int, rebuilds: int, mode: str,
-                   keep_keys: bool = False) -> int:
+                   keep_keys: bool = False, particles: int = 0) -> int:
     """Kernels launched over `half_steps` half steps with `rebuilds` list rebuilds
-    (keep_keys: a batch with per-instance decisions, one more kernel per rebuild)."""
+    (keep_keys: a batch with per-instance decisions, one more kernel per rebuild; particles: with
+    that many and neighbour lists, 0: the cell list and list build alone, marked and filled)."""
     bits = 1
     while bits < 31 and (1 << bits) < num_cells:
         bits += 1
@@ -195,6 +196,10 @@ def count_launches(num_cells: int, half_steps: int, rebuilds: int, mode: str,
     # and the neighbour-list build.  In gated mode the rebuild kernels are launched every
     # half step (and return at once when the lists are kept).
     rebuild_kernels = 3 * passes + 7 + (1 if keep_keys else 0)
+    if particles:
+        # the four kernels of the work order; grids with a cell or more per particle get their
+        # cell starts from one kernel instead of three
+        rebuild_kernels += 4 - (2 if num_cells >= particles else 0)
     if mode == "gated":
         return half_steps * (3 + rebuild_kernels)
     return 3 * half_steps + rebuilds * rebuild_kernels
@@ -560,8 +565,8 @@ def batch_measure(n_inst: int, precision: str, args, stream, steps: int, warmup:
         return {"min": int(c.min()), "mean": float(c.mean()), "max": int(c.max())}
 
     sol = make_solver()
-    lanes = lanes_in_effect(sol)
     sol.upload_instances(mine, stream=stream)
+    lanes = lanes_in_effect(sol)  # the default block size follows the number of particles
     sol.step(warmup, stream=stream)
     torch.cuda.synchronize()
     r0 = sol.rebuild_count(stream=stream)
@@ -595,7 +600,7 @@ def batch_measure(n_inst: int, precision: str, args, stream, steps: int, warmup:
            "list_rebuilds": {"timed": rebuilds, "half_steps": 2 * steps},
            "gpu_launches": count_launches(
                sol_cells_batch(p, n_inst, skin, lanes["cell_divisions"]), 2 * steps,
-               rebuilds, args.graph_mode, own),
+               rebuilds, args.graph_mode, own, particles=n),
            "autotune": None}
     if tuned:
         from tmp_sph_gb300 import autotune
@@ -915,8 +920,8 @@ def main():
 
     sol = S.Solver(p, n, precision=args.precision)
     configure(sol)
-    lanes = lanes_in_effect(sol)
     sol.upload(st["pos"], st["vel"], st["rho"], st["p"], st["type"], stream=stream)
+    lanes = lanes_in_effect(sol)  # the default block size follows the number of particles
 
     def barrier():
         if ws > 1:
@@ -1132,7 +1137,8 @@ def main():
         "drop_in_step_loop": dropin,
         "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "steps": args.e2e_steps},
-        "gpu_launches": count_launches(sol_cells, 2 * args.steps, rebuilds, args.graph_mode),
+        "gpu_launches": count_launches(sol_cells, 2 * args.steps, rebuilds, args.graph_mode,
+                                       particles=n),
         "list_rebuilds": {"timed": rebuilds, "half_steps": 2 * args.steps,
                           "skin_permille": args.skin, "list_skin_over_kh_at_end": skin_end},
         "configured_run": run,

@@ -25,13 +25,15 @@
 // support radius, and the lanes of a warp (particles of two or three adjacent cells) almost
 // always have at least one hit per candidate, so a pass that tests and evaluates in one loop
 // pays the full pair body for every candidate.  k_nbr_build therefore walks the candidates
-// once per list build and stores the hits of particle i, in walk order, in column i of its
-// warp's slot block (nbr_col); both passes then iterate only true neighbours, in the same
-// order, so the sums are the same as a walking pass.  The passes are limited by L1 data-stage
-// wavefronts (each lane gathers a different record): interleaving the slots (in groups of four
-// per lane) makes a warp's list read four lines per four steps instead of one line per lane
-// and step.  A particle with more hits than
-// the list capacity is marked and walks the cells itself (same order again).
+// once per list build and stores the hits of the particle at work position t (all fluid slots
+// first, then the walls; NbrList::order), in walk order, in column t of its warp's slot block
+// (nbr_col); both passes then iterate only true neighbours, in the same order, so the sums are the
+// same as a walking pass.  The passes wait for the gathers (each lane another record): the slots
+// are interleaved in groups of four per lane, so that a warp's list read touches four lines per
+// four steps, and padded to whole groups, so that the four gathers of a group are issued together
+// without a branch.  Large FP32 runs share each list and gather between two particles
+// (ns_twin.cu).  A particle with more hits than the list capacity is marked and walks the cells
+// itself (same order again).
 //
 // With a Verlet skin the list is built with the cutoff kh(1 + s) (NbrList::cut2, else
 // kh2_list) on cells kh(1 + skin) wide, s <= skin, and kept while the displacements since the

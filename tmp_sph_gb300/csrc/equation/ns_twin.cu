@@ -15,9 +15,10 @@
 // records apart: 17 wavefronts, and pass 1 at 467 instead of 361 us (4.96M particles).
 //
 // Measured, pass 1 / pass 2 against one particle per thread with one gather in flight: 4.96M
-// particles 520 / 609 -> 361 / 582 us, a disordered surge of 6.70M 1020 / 1078 -> 750 / 927 us.
-// What is left is latency: pass 2 issues in 60-70% of cycles with 18 warps per SM (104 registers),
-// L1 data stage 45% (pass 1 70%).  Slower: 80 registers (630 us, the gathers of a chunk no longer
+// particles 520 / 609 -> 361 / 582 us, a disordered surge of 6.70M 1020 / 1078 -> 750 / 927 us (with
+// the copies that pass 2 no longer writes, 357 / 555 of 4.96M).  What is left is latency: pass 2
+// issues in 62% of cycles with 19 warps per SM (a cap of 104 registers, 96 used), L1 data stage 48%
+// (pass 1: 60%, 22 warps, 73%).  Slower: 80 registers (630 us, the gathers of a chunk no longer
 // issued together), records of the next half chunk loaded during the current one (640-690 us),
 // lists prefetched into L2 ahead of their use (level).
 #include <cuda_runtime.h>

@@ -150,13 +150,14 @@ using Pass1Out = Pass1OutT<float>;
 
 enum HalfStep { HALF_PREDICT = 0, HALF_CORRECT = 1 };
 
-// Neighbour list: slot c of particle i at idx[(i / 32) * cap * 32 + (c / 4) * 128 + (i % 32) * 4
-// + c % 4] (each warp of 32 consecutive particles owns a block of cap x 32 slots, its particles'
-// slots four to an int4, side by side), count[i] entries, and xb[i]
-// the position i had when the list was built (its record position).  The list
-// holds every pair closer than the list cutoff (KParams::kh2_list, the support radius plus a
-// skin), in candidate-walk order; count[i] > cap means the list overflowed for i and the
-// passes walk the cells for it instead.  With cell codes (kCodes) a slot holds the index above six
+// Neighbour list: slot c of work position t at idx[(t / 32) * cap * 32 + (c / 4) * 128 + (t % 32) * 4
+// + c % 4] (each warp of 32 consecutive positions owns a block of cap x 32 slots, its particles'
+// slots four to an int4, side by side; the last int4 filled up with the padding slot n), count[t]
+// entries, and xb[i] the position slot i had when the list was built (its record position).  The
+// list holds every pair closer than the list cutoff (KParams::kh2_list, the support radius plus a
+// skin), in candidate-walk order; count[t] > cap means the list overflowed for that particle and the
+// passes walk the cells for it instead.  Lists shared by two particles (ns_twin.cu) have one column
+// per thread in the same form.  With cell codes (kCodes) a slot holds the index above six
 // bits with the neighbour's anchor relative to i's ((dz+1) << 4 | (dy+1) << 2 | (dx+1)), from
 // which the passes rebuild relative positions out of the cell-local offsets.
 struct NbrList {

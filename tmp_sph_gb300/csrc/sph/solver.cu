@@ -5,7 +5,7 @@
 // SPH_NS, PC_prediction, recover, then the same for PC_correction).  Here one half step is
 //
 //   rebuild decision  ->  [radix sort (cell key, slot)  ->  gather y -> x -> y in cell order
-//   + dense cell starts  ->  neighbour-list build (y)]  ->  pass 1 (y -> records p1)
+//   + dense cell starts  ->  work order  ->  neighbour-list build (y)]  ->  pass 1 (y -> records p1)
 //   ->  pass 2 + integrator (p1 -> y in place, next cell keys, displacement box)
 //
 // so the state never returns to original order inside a step (the original particle id
@@ -308,7 +308,7 @@ template <class P>
 constexpr bool kTwin = P::kId == SPH_PREC_FP32 || P::kId == SPH_PREC_MIXED_ABS;
 
 // Threads per block of the neighbour kernels: the option, or by default 64 with two particles per
-// thread (104 registers a thread: nine blocks per SM; 128 threads: pass 2 596 against 582 us at
+// thread (pass 2 takes 96 registers: ten blocks per SM; 128 threads: pass 2 596 against 582 us at
 // 4.96M particles), 32 in FP64 (its pipe bounds a pass, so the SMs should get equal shares of warps:
 // 133,968 particles, three steps 6.56 ms with 128, 6.28 with 32; 27,288 particles 3.29 and 2.97),
 // else 256 in FP32 up to 60,000 particles and 128 above, where whole blocks of 256 leave SMs
