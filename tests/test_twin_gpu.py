@@ -54,6 +54,9 @@ def run(st, p, opts, precision="fp32", steps=3, instances=0):
     ("fp32", True, {"SPH_OPT_CELL_DIVISIONS": 2, "SPH_OPT_CONDITIONAL_GRAPH": 0}),
     ("fp32", True, {"SPH_OPT_CELL_DIVISIONS": 1, "SPH_OPT_PASS1_LANES": 1}),
     ("fp32", True, {"SPH_OPT_NEIGHBOR_CAP": 80}),  # some lists overflow and walk the cells
+    ("fp32", True, {"SPH_OPT_NEIGHBOR_CAP": 80, "SPH_OPT_CELL_DIVISIONS": 1,  # both of a cell walk
+                    "SPH_OPT_PASS1_LANES": 1}),
+    ("mixed_abs", True, {"SPH_OPT_NEIGHBOR_CAP": 16, "SPH_OPT_CELL_DIVISIONS": 1}),
     ("fp32", True, {"SPH_OPT_BLOCK_THREADS": 256}),
 ])
 def test_twin_gives_the_bits_of_one_particle_per_thread(sphlib, cuda, precision, disorder, opts):
