@@ -322,25 +322,47 @@ __device__ __forceinline__ void visit_twin(const NbrList& nl, const float4* __re
     });
 }
 
-// The same over the cells, for two particles of one cell that overflowed their list: the candidates of
-// a row of cells four at a time, the last four filled up with the padding record n.  Bound by the
-// latency of one candidate's arithmetic after another, on few warps: 32,000 particles at one point
-// among 765,828 take 13.2 ms a step; 48.7 with the two walked one after the other, a candidate at a
-// time, 41.3 with one particle per thread.
+// The cells of two particles that overflowed their list, when they are of one cell or of neighbouring
+// ones: one box of cells holds the walks of both, and a candidate that only one of them walks lies
+// outside the other's support radius.
+struct TwinCells {
+    int xl, xh, yl, yh, zl, zh;
+    bool near;
+};
+__device__ __forceinline__ TwinCells twin_cells(const KParamsT<float>& k,
+                                                const unsigned* __restrict__ keys, const Twin& tw) {
+    TwinCells w;
+    const unsigned ka = keys[tw.a], kb = keys[tw.b];
+    w.near = !inactive_key(k, ka) && !inactive_key(k, kb);
+    if (!w.near) return w;
+    int ax, ay, az, bx, by, bz;
+    cell_of_key(k.gx, k.gy, ka, ax, ay, az);
+    cell_of_key(k.gx, k.gy, kb, bx, by, bz);
+    const int r = k.reach;
+    w.near = abs(ax - bx) <= 1 && abs(ay - by) <= 1 && abs(az - bz) <= 1;
+    w.xl = max(min(ax, bx) - r, 0), w.xh = min(max(ax, bx) + r, k.gx - 1);
+    w.yl = max(min(ay, by) - r, 0), w.yh = min(max(ay, by) + r, k.gy - 1);
+    w.zl = max(min(az, bz) - r, 0), w.zh = min(max(az, bz) + r, k.gz - 1);
+    return w;
+}
+
+// one(a, v) for the records of those cells, the candidates of a row of cells four at a time, the last
+// four filled up with the padding record n.  Bound by the latency of one candidate's arithmetic after
+// another, on few warps: 32,000 particles at one point among 765,828 take 13.2 ms a step; 48.7 with
+// the two walked one after the other, a candidate at a time, 41.3 with one particle per thread.  With
+// 64 list slots, which most fluid particles overflow, 1.46 ms (1.76, 1.23; on cells of the cutoff 1.52
+// against 1.80); passing over candidates that neither needs costs the list path its registers.
 template <class F>
 __device__ __forceinline__ void walk_twin(const KParamsT<float>& k, const int* __restrict__ cs,
-                                          unsigned key, const float4* __restrict__ R, F&& one) {
-    if (inactive_key(k, key)) return;
-    int cx, cy, cz;
-    cell_of_key(k.gx, k.gy, key, cx, cy, cz);
-    const int r = k.reach, xl = max(cx - r, 0), xh = min(cx + r, k.gx - 1);
+                                          const TwinCells& w, const float4* __restrict__ R,
+                                          F&& one) {
 #pragma unroll 1
-    for (int z = max(cz - r, 0); z <= min(cz + r, k.gz - 1); z++) {
+    for (int z = w.zl; z <= w.zh; z++) {
 #pragma unroll 1
-        for (int y = max(cy - r, 0); y <= min(cy + r, k.gy - 1); y++) {
+        for (int y = w.yl; y <= w.yh; y++) {
             const int row = (z * k.gy + y) * k.gx;
-            const int j0 = max(__ldg(cs + row + xl), 0);
-            const int j1 = min(__ldg(cs + row + xh + 1), k.n);  // bounds guard only
+            const int j0 = max(__ldg(cs + row + w.xl), 0);
+            const int j1 = min(__ldg(cs + row + w.xh + 1), k.n);  // bounds guard only
 #pragma unroll 1
             for (int j = j0; j < j1; j += 4) {
                 float4 a[4], v[4];
@@ -434,23 +456,26 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
                 if (!B.fi && r2 < k.kh2) B.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
             });
         }
-    } else if (A.fi && B.fi && keys[tw.a] == keys[tw.b]) {
-        walk_twin(k, cs, keys[tw.a], in.rec, [&](const float4& aj, const float4& vj) {
-            pass1_twin<P>(k, A, B, aj, vj);
-        });
     } else {
-#pragma unroll 1
-        for (int m = 0; m < 2; m++) {
-            Pass1Acc<P> C = m ? B : A;
-            walk_pairs<P, 2>(k, cs, keys, in.rec, m ? tw.b : tw.a, C.pi, k.kh2,
-                             [&](int j, unsigned, const float4&, float dx, float dy, float dz,
-                                 float r2) {
-                float4 aj, vj;
-                ld_rec(in.rec, j, aj, vj);
-                C.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
+        const TwinCells w = twin_cells(k, keys, tw);
+        if (w.near && A.fi && B.fi) {
+            walk_twin(k, cs, w, in.rec, [&](const float4& aj, const float4& vj) {
+                pass1_twin<P>(k, A, B, aj, vj);
             });
-            if (m) B = C;
-            else A = C;
+        } else {
+#pragma unroll 1
+            for (int m = 0; m < 2; m++) {
+                Pass1Acc<P> C = m ? B : A;
+                walk_pairs<P, 2>(k, cs, keys, in.rec, m ? tw.b : tw.a, C.pi, k.kh2,
+                                 [&](int j, unsigned, const float4&, float dx, float dy, float dz,
+                                     float r2) {
+                    float4 aj, vj;
+                    ld_rec(in.rec, j, aj, vj);
+                    C.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
+                });
+                if (m) B = C;
+                else A = C;
+            }
         }
     }
     A.template finish<false>(k, out, nullptr, nullptr, tw.a);
@@ -476,24 +501,27 @@ k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
                 visit_twin(nl, p1.nrec, u, cnt, [&](const float4& aj, const float4& vj) {
                     pass2_twin<P, MODE>(k, A, B, aj, vj);
                 });
-            } else if (A.active && B.active && keys[tw.a] == keys[tw.b]) {
-                walk_twin(k, cs, keys[tw.a], p1.nrec, [&](const float4& aj, const float4& vj) {
-                    pass2_twin<P, MODE>(k, A, B, aj, vj);
-                });
             } else {
+                const TwinCells w = twin_cells(k, keys, tw);
+                if (w.near && A.active && B.active) {
+                    walk_twin(k, cs, w, p1.nrec, [&](const float4& aj, const float4& vj) {
+                        pass2_twin<P, MODE>(k, A, B, aj, vj);
+                    });
+                } else {
 #pragma unroll 1
-                for (int m = 0; m < 2; m++) {
-                    Pass2Acc<P, MODE> C = m ? B : A;
-                    if (C.active)
-                        walk_pairs<P, 2>(k, cs, keys, p1.nrec, m ? tw.b : tw.a, C.pi, k.kh2,
-                                         [&](int j, unsigned, const float4&, float dx, float dy,
-                                             float dz, float r2) {
-                            float4 aj, vj;
-                            ld_rec(p1.nrec, j, aj, vj);
-                            C.pair(k, p1, j, aj, vj, dx, dy, dz, r2, 0.f);
-                        });
-                    if (m) B = C;
-                    else A = C;
+                    for (int m = 0; m < 2; m++) {
+                        Pass2Acc<P, MODE> C = m ? B : A;
+                        if (C.active)
+                            walk_pairs<P, 2>(k, cs, keys, p1.nrec, m ? tw.b : tw.a, C.pi, k.kh2,
+                                             [&](int j, unsigned, const float4&, float dx, float dy,
+                                                 float dz, float r2) {
+                                float4 aj, vj;
+                                ld_rec(p1.nrec, j, aj, vj);
+                                C.pair(k, p1, j, aj, vj, dx, dy, dz, r2, 0.f);
+                            });
+                        if (m) B = C;
+                        else A = C;
+                    }
                 }
             }
         }
