@@ -216,7 +216,7 @@ __device__ __forceinline__ bool inside(double r2, double cut2) {
 
 // Pair arithmetic: in FP32 the distance and the reciprocal of a pair come from the hardware's
 // approximate instructions (sqrt.approx, rcp.approx: within about one ulp, instead of the
-// correctly rounded sequences); FP64 keeps correctly rounded sqrt and division.  The .ftz
+// correctly rounded sequences), in FP64 from its own refinement of them (below).  The .ftz
 // forms flush subnormal inputs and results to zero, which no pair meets (the arguments are a
 // density near rho0, r^2 + eta^2 >= eta^2, and r^2, which is 0 for coincident particles and
 // otherwise many decades above the subnormal range), and so give the same value as the plain
