@@ -53,7 +53,8 @@ __device__ __forceinline__ size_t twin_col(const NbrList& nl, int u) {
     return (size_t)(u >> 5) * ((size_t)nl.cap << 6) + ((size_t)(u & 31) << 2);
 }
 // nl.count of a thread: the entries of its shared list; TWIN_WALKS when one of its particles
-// overflowed; below that, of two instances, the chunks of its particles' own lists (split_count).
+// overflowed or the two do not fit it; below that, of two instances, the chunks of its particles' own
+// lists (split_count).
 constexpr int TWIN_WALKS = -1;
 constexpr int SPLIT_BITS = 15;
 __device__ __forceinline__ int split_count(int chunks_a, int chunks_b) {
@@ -357,7 +358,8 @@ k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __rest
         [&]() { w.drain(); });
     w.flush(pad_slot<P>(k.n));
     // a particle overflows when its own neighbours do, which the shared list may hold: counted only
-    // when the shared list is longer than one particle's room
+    // when the shared list is longer than one particle's room.  Two full lists with nothing in common
+    // do not fit it with the particles themselves: they walk without having overflowed.
     bool over = false;
     if (w.cnt > nl.cap) {
         int na = 0, nb = 0;
@@ -370,9 +372,9 @@ k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __rest
                 nb += j != b && r2b < (fj ? cut2 : cb);
             },
             [] {});
-        over = na > nl.cap || nb > nl.cap || w.cnt > 2 * nl.cap;
+        over = na > nl.cap || nb > nl.cap;
     }
-    nl.count[u] = over ? TWIN_WALKS : w.cnt;
+    nl.count[u] = over || w.cnt > 2 * nl.cap ? TWIN_WALKS : w.cnt;
     raise_flags(err, over ? SPH_FLAG_NEIGHBOR_OVERFLOW : 0u);
 }
 
