@@ -258,7 +258,7 @@ cudaError_t launch_gather(const KParamsT<typename P::T>& k, const int* perm,
                           const ParticleSetT<typename P::T>& src, ParticleSetT<typename P::T> dst,
                           int with_tmp, int dense, const unsigned* keys, cudaStream_t s,
                           const unsigned* gate = nullptr);
-// Recompute the cell keys of `set` on the grid of `k` (k.n particles).
+// Recompute the cell keys of `set` on the grid of `k` (k.n particles), and FP64 pair volumes.
 template <class P>
 cudaError_t launch_rehash(const KParamsT<typename P::T>& k, const ParticleSetT<typename P::T>& set,
                           unsigned* hash, unsigned* err, cudaStream_t s);

@@ -800,7 +800,8 @@ __global__ void k_upload_sorted(KParamsT<typename P::T> kp, const float* __restr
     reduce_disp(kp, box, disp, s_box, s_inst);
 }
 
-// Cell keys of a resident set on the current grid (after the grid changed under it).
+// Cell keys of a resident set on the current grid, and in FP64 the pair volumes of its records (after
+// the grid or the parameters changed under it).
 template <class P>
 __global__ void k_rehash(KParamsT<typename P::T> kp, ParticleSetT<typename P::T> set,
                          unsigned* __restrict__ hash, unsigned* err) {
@@ -816,6 +817,8 @@ __global__ void k_rehash(KParamsT<typename P::T> kp, ParticleSetT<typename P::T>
         const auto q = set.rec[2 * (size_t)i];
         hash[i] = slot_key(kp, inst, fluid, q.x, q.y, q.z, &f);
     }
+    if constexpr (std::is_same<typename P::T, double>::value)
+        set.vol[i] = pair_volume(kp, fabs(set.rec[2 * (size_t)i + 1].w));
     raise_flags(err, f);
 }
 

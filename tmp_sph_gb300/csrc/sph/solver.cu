@@ -1310,8 +1310,8 @@ static int step_impl(sph_ctx* c, int nsteps, void* stream) {
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (c->rehash) {
-        // the grid changed (sph_set_params, skin option): the keys pass 2 wrote for the
-        // current positions index the old grid
+        // the grid or the parameters changed (sph_set_params, skin option): the keys pass 2 wrote
+        // for the current positions index the old grid, FP64's pair volumes hold the old mass and h
         const cudaError_t e = with_prec(c, [&](auto tag) {
             using P = decltype(tag);
             return launch_rehash<P>(resident_kparams<typename P::T>(c), State<P>::y(c), c->hash_x,
