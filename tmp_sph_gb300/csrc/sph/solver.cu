@@ -1459,9 +1459,12 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
         return SPH_ERR_CUDA;
     if (build_cell_starts(c->keys_sorted, n, c->P.num_cells, c->cell_start, s) != cudaSuccess)
         return SPH_ERR_CUDA;
-    // the drop-in builds and uses its list within this call, with the constant cutoff
+    // the drop-in builds and uses its list within this call, for every particle and with the constant
+    // cutoff, whatever the resident lists last were
     NbrList dl = c->nl;
     dl.cut2 = nullptr;
+    dl.iw = nullptr;
+    dl.inst = nullptr;
     dl.rank = nullptr;
     dl.order = nullptr;
     const NbrList* nl = list_for(c) ? &dl : nullptr;
