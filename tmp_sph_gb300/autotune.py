@@ -17,8 +17,8 @@ once the box of all displacements has a half-diagonal of skin kh / 2, which such
 after moving skin kh).  v defaults to the dam-break surge-front speed 2 sqrt(g H) of the
 tallest water column H.  The search is staged: the launch shape (threads, particles per
 thread, pass-1 lanes) at the default skin and cell size, then skin and cell size for the best
-shape.  The model's best few and the library default are then run for `confirm_steps` steps
-each (adaptive skin on, as the solver runs them) and the fastest measured wins if it beats the
+shape.  The model's best few and the library default (threads 0: the block size the solver picks
+by precision and particle count) are then run for `confirm_steps` steps each (adaptive skin on, as the solver runs them) and the fastest measured wins if it beats the
 default by at least `margin` (1%; closer than that the two are within run-to-run noise and the
 default stays), so the choice is not slower than the default on the workload it was tuned on.
 
@@ -34,7 +34,7 @@ import math
 from . import api
 from . import solver as S
 
-THREADS = (64, 128, 256)
+THREADS = (32, 64, 128, 256)
 PPT = (1, 2, 4)
 LANES = (1, 2, 4)
 SKINS = (0, 50, 100, 150, 200, 300)
@@ -103,12 +103,17 @@ def step_cost(m: dict, p, v: float) -> float:
 
 
 def default_choice(precision: str) -> dict:
-    """The library's default: with the FP32 pair arithmetic (FP32, and mixed precision on FP32
-    positions) 256 threads and cells of a third of the list cutoff, otherwise 128 threads and
-    cells of the cutoff; one pass-1 lane, one particle per thread and skin 0.1 kh in all."""
+    """The library's default cell size, skin, lanes and particles per thread, and the block size of
+    its small runs (FP32 pair arithmetic: 256 threads; otherwise 128): where the search starts.  The
+    solver's own block size depends on the particle count as well (library_default)."""
     fp32 = precision in ("fp32", "mixed_abs")
     return {"threads": 256 if fp32 else 128, "ppt": 1, "lanes": 1,
             "skin_permille": DEFAULT_SKIN, "divisions": 3 if fp32 else 1}
+
+
+def library_default(precision: str) -> dict:
+    """The library's default as a choice to run: threads 0 leaves the block size to the solver."""
+    return {**default_choice(precision), "threads": 0}
 
 
 def _key(m: dict) -> tuple:
@@ -145,15 +150,15 @@ def tune(p, states, *, precision: str = "fp32", threads=THREADS, ppt=PPT, skins=
          lanes=LANES, divisions=DIVISIONS, speed: float | None = None,
          confirm_steps: int = 100, confirm_top: int = 3, margin: float = 0.01) -> dict:
     """Best (threads, ppt, lanes, skin, divisions) for this workload; `states` is one state dict
-    or a list of them (batched instances).  Returns the choice with the measured table and the
-    confirmation runs."""
+    or a list of them (batched instances).  Returns the choice (threads 0: the solver's own) with the
+    measured table and the confirmation runs."""
     import torch
     states = states if isinstance(states, list) else [states]
     n = sum(len(st["rho"]) for st in states)
     v = speed if speed is not None else surge_speed(states, float(p.gravity))
     stream = torch.cuda.Stream()
     table = []
-    dflt = default_choice(precision)
+    dflt = library_default(precision)
     skin0 = dflt["skin_permille"] if dflt["skin_permille"] in skins else skins[0]
     div0 = dflt["divisions"] if dflt["divisions"] in divisions else divisions[0]
     with S.Solver(p, n, precision=precision) as sol:
