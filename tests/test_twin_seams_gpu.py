@@ -28,6 +28,18 @@ def with_fluid(pos, dx, seed=0):
     return out, p
 
 
+def cluster(size, dx):
+    """`size` particles on a lattice 1.91 dx across: all within one support radius (2.6 dx)."""
+    m = int(np.ceil(size ** (1 / 3)))
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:size]
+    return 1.91 * dx * g / (np.sqrt(3) * (m - 1))
+
+
+def heavy_drop(b, dx):
+    """A drop at nearly the same place in every instance whose particles have 100 neighbours each."""
+    return np.array([0.4, 0.2, 0.3]) + cluster(101 - b % 2, dx) + [0, 0, dx * (b % 3)]
+
+
 def drop(b, dx):
     """A drop of 27 particles (28 or 26 in some instances, so that both parities of the seams occur)
     at nearly the same place in every instance."""
@@ -82,14 +94,15 @@ def test_instances_stay_apart(sphlib, cuda, kind, precision):
             assert np.array_equal(out[k][off[b]:off[b + 1]], ref[k]), (b, k)
 
 
-@pytest.mark.parametrize("opts", [{}, {"SPH_OPT_NEIGHBOR_CAP": 16},
-                                  {"SPH_OPT_CELL_DIVISIONS": 1, "SPH_OPT_PASS1_LANES": 1}])
-def test_seams_give_the_bits_of_one_particle_per_thread(sphlib, cuda, opts):
+@pytest.mark.parametrize("kind,opts", [(drop, {}), (heavy_drop, {"SPH_OPT_NEIGHBOR_CAP": 96}),
+                                       (drop, {"SPH_OPT_CELL_DIVISIONS": 1,
+                                               "SPH_OPT_PASS1_LANES": 1})])
+def test_seams_give_the_bits_of_one_particle_per_thread(sphlib, cuda, kind, opts):
     """The same batches at the default skin, with lists that overflow at the seams, and on cells of
     the cutoff: fields and flags of one particle per thread."""
     from tmp_sph_gb300 import api
     o = {getattr(api, k): v for k, v in opts.items()}
-    states, p = batch_of(drop)
+    states, p = batch_of(kind)
     two, _ = run_batch(states, p, o, "fp32", steps=4)
     one, _ = run_batch(states, p, {**o, api.SPH_OPT_PARTICLES_PER_THREAD: 2}, "fp32", steps=4)
     assert two["flags"] == one["flags"]

@@ -52,9 +52,8 @@ __device__ __forceinline__ Twin twin_of(const NbrList& nl, int u, int n) {
 __device__ __forceinline__ size_t twin_col(const NbrList& nl, int u) {
     return (size_t)(u >> 5) * ((size_t)nl.cap << 6) + ((size_t)(u & 31) << 2);
 }
-// nl.count of a thread: the entries of its shared list; TWIN_WALKS when one of its particles
-// overflowed or the two do not fit it; below that, of two instances, the chunks of its particles' own
-// lists (split_count).
+// nl.count of a thread: the entries of its shared list; TWIN_WALKS when they do not fit it; below that,
+// of two instances, the chunks of its particles' own lists (split_count).
 constexpr int TWIN_WALKS = -1;
 constexpr int SPLIT_BITS = 15;
 __device__ __forceinline__ int split_count(int chunks_a, int chunks_b) {
@@ -357,24 +356,36 @@ k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __rest
         },
         [&]() { w.drain(); });
     w.flush(pad_slot<P>(k.n));
-    // a particle overflows when its own neighbours do, which the shared list may hold: counted only
-    // when the shared list is longer than one particle's room.  Two full lists with nothing in common
-    // do not fit it with the particles themselves: they walk without having overflowed.
+    // A particle overflows when its own neighbours do: counted only when the shared list is longer than
+    // one particle's room, from the list just written where it is whole (a third of the candidates of
+    // another walk), else from the candidates.  Only a list that is not whole sends its particles to
+    // their cells: a whole one has both, overflowed or not (765,828 particles with 80 slots, of which a
+    // few have more, 0.88 ms a step when those walked, 0.30 now; 0.33 with one particle per thread).
     bool over = false;
     if (w.cnt > nl.cap) {
         int na = 0, nb = 0;
-        visit(
-            [&](int j, const float4& p) {
-                float r2a, r2b;
-                dist(p, r2a, r2b);
-                const bool fj = fluid_rec(p.w);
-                na += j != a && r2a < (fj ? cut2 : ca);
-                nb += j != b && r2b < (fj ? cut2 : cb);
-            },
-            [] {});
+        auto count = [&](int j, const float4& p) {
+            float r2a, r2b;
+            dist(p, r2a, r2b);
+            const bool fj = fluid_rec(p.w);
+            na += j != a && r2a < (fj ? cut2 : ca);
+            nb += j != b && r2b < (fj ? cut2 : cb);
+        };
+        if (w.cnt <= 2 * nl.cap) {
+#pragma unroll 1
+            for (int c = 0; c < w.cnt; c += 4) {
+                const int4 q = *reinterpret_cast<const int4*>(w.col + ((size_t)c << 5));
+                const int e[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int l = 0; l < 4; l++)
+                    if (c + l < w.cnt) count(e[l], ld_pos(X, (size_t)e[l]));
+            }
+        } else {
+            visit(count, [] {});
+        }
         over = na > nl.cap || nb > nl.cap;
     }
-    nl.count[u] = over || w.cnt > 2 * nl.cap ? TWIN_WALKS : w.cnt;
+    nl.count[u] = w.cnt > 2 * nl.cap ? TWIN_WALKS : w.cnt;
     raise_flags(err, over ? SPH_FLAG_NEIGHBOR_OVERFLOW : 0u);
 }
 
@@ -414,7 +425,7 @@ __device__ __forceinline__ void visit_split(const KParamsT<float>& k, const NbrL
     });
 }
 
-// The cells of two particles that overflowed their list, when they are of one cell or of neighbouring
+// The cells of two particles that do not fit their list, when they are of one cell or of neighbouring
 // ones: one box of cells holds the walks of both, and a candidate that only one of them walks lies
 // outside the other's support radius.  (Never two instances: empty layers lie between their cells.)
 struct TwinCells {
@@ -441,9 +452,8 @@ __device__ __forceinline__ TwinCells twin_cells(const KParamsT<float>& k,
 // one(a, v) for the records of those cells, the candidates of a row of cells four at a time, the last
 // four filled up with the padding record n.  Bound by the latency of one candidate's arithmetic after
 // another, on few warps: 32,000 particles at one point among 765,828 take 13.2 ms a step; 48.7 with
-// the two walked one after the other, a candidate at a time, 41.3 with one particle per thread.  With
-// 64 list slots, which most fluid particles overflow, 1.46 ms (1.76, 1.23; on cells of the cutoff 1.52
-// against 1.80); passing over candidates that neither needs costs the list path its registers.
+// the two walked one after the other, a candidate at a time, 41.3 with one particle per thread.  Passing
+// over candidates that neither needs costs the list path its registers.
 template <class F>
 __device__ __forceinline__ void walk_twin(const KParamsT<float>& k, const int* __restrict__ cs,
                                           const TwinCells& w, const float4* __restrict__ R,
