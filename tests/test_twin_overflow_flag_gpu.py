@@ -33,3 +33,18 @@ def test_flag_and_fields_of_full_lists(sphlib, cuda, precision, size, over):
     assert two["flags"] == one["flags"]
     for k in KEYS:
         assert np.isfinite(one[k]).all() and np.array_equal(two[k], one[k]), k
+
+
+@pytest.mark.parametrize("slots", [16, 80, 96, 112])
+def test_capacities_either_side_of_the_rule(sphlib, cuda, slots):
+    """A disordered flow with lists most particles overflow (one particle per thread) and lists most
+    fit (two): the fields and flags of one particle per thread."""
+    from test_twin_gpu import state
+    from tmp_sph_gb300 import api
+    st, p = state(0.0061, True)
+    o = {api.SPH_OPT_NEIGHBOR_CAP: slots}
+    two = run(st, p, o)
+    one = run(st, p, {**o, api.SPH_OPT_PARTICLES_PER_THREAD: 2})
+    assert two["flags"] == one["flags"]
+    for k in KEYS:
+        assert np.array_equal(two[k], one[k]), k

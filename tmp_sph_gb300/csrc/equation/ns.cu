@@ -517,11 +517,14 @@ void pass2_launch(const KParamsT<typename P::T>& k, const ParticleSetT<typename 
 
 }  // namespace
 
+double lattice_neighbours(const sph_params& p, double skin) {
+    const double r = (double)p.kh * (1.0 + skin) / (double)p.dx;
+    return 4.18879020478639 * r * r * r;
+}
+
 int nbr_capacity_for(const sph_params& p, double skin) {
     // 1.5x the particles of a lattice inside the list sphere, rounded up to 16
-    const double r = (double)p.kh * (1.0 + skin) / (double)p.dx;
-    const double lattice = 4.18879020478639 * r * r * r;
-    int cap = (int)(1.5 * lattice) + 16;
+    int cap = (int)(1.5 * lattice_neighbours(p, skin)) + 16;
     cap = (cap + 15) & ~15;
     return cap < 32 ? 32 : cap;
 }

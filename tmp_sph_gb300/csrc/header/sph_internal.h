@@ -181,6 +181,8 @@ struct NbrList {
     // the list columns and counts are indexed by t; NULL: slot t
     const int* order = nullptr;
 };
+// Particles of a lattice of spacing dx within kh (1 + skin) of a point.
+double lattice_neighbours(const sph_params& p, double skin);
 // List slots per particle: 1.5x the lattice particles within kh (1 + skin), rounded up to 16.
 int nbr_capacity_for(const sph_params& p, double skin = 0.0);
 

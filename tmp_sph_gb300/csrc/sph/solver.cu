@@ -295,14 +295,26 @@ static bool fp32_pairs(int prec) { return prec == SPH_PREC_FP32 || prec == SPH_P
 
 // Whether the lists and passes take two particles per thread (equation/ns_twin.cu): the FP32 pair
 // arithmetic, one pass-1 lane, the default of one particle per thread, one rebuild decision for
-// all slots, and enough particles to fill the GPU with half the threads: at 380,000 particles the
-// two forms are level (5 steps 0.93 ms against 0.89 in a calm flow, 1.11 against 1.18 in a
-// disordered one), at 200,000 one particle per thread wins (0.70 against 0.57), at 766,000 two do
-// (1.60 against 1.75).  Both give the same bits.
+// all slots, lists that most particles fit (twin_room), and enough particles.  The count is of all
+// particles (how many are fluid is known on the device only), of which the walls do little in a pass:
+// of 458,244 with 265,188 fluid the two forms are level in a calm flow (a step 0.197 ms either way) and
+// two win in a disordered one (0.348 against 0.374); with 15,625 fluid of 459,133 one would win (0.113
+// against 0.078).  At 380,000 (the 60% fluid of a dam break) they are level (5 steps 0.93 ms against
+// 0.89, disordered 1.11 against 1.18), at 200,000 one wins (0.70 against 0.57).  Without a skin the
+// builds of every half step favour one up to about a million (458,244: 0.82 against 0.66).  Both give
+// the same bits.
 constexpr int TWIN_MIN_PARTICLES = 400000;
+// Whether the list capacity holds the lists of a flow: a tenth more than a lattice has within kh.  Two
+// particles that do not fit walk their cells together with the others of their warp.  765,828 particles
+// (74 in the lattice sphere), two per thread against one: 96 slots 0.30 against 0.33 ms a step,
+// disordered 0.51 against 0.68; 80 slots 0.88 against 0.33 and 1.01 against 1.64; 48 slots 1.69 against
+// 1.27 and 2.46 against 1.53.  With h = 1.5 dx (113): 128 slots 0.50 against 0.53 and 1.42 against 2.41.
+static bool twin_room(const sph_ctx* c) {
+    return c->nl.idx && c->nl.cap >= 1.1 * lattice_neighbours(c->P, 0.0);
+}
 static bool twin_lists(const sph_ctx* c) {
-    return fp32_pairs(c->prec) && c->opt_nbr_list && c->nl.idx && pass1_lanes(c) == 1 &&
-           c->opt_ppt == 1 && !per_instance(c) && c->n >= TWIN_MIN_PARTICLES;
+    return fp32_pairs(c->prec) && c->opt_nbr_list && pass1_lanes(c) == 1 && c->opt_ppt == 1 &&
+           !per_instance(c) && c->n >= TWIN_MIN_PARTICLES && twin_room(c);
 }
 template <class P>
 constexpr bool kTwin = P::kId == SPH_PREC_FP32 || P::kId == SPH_PREC_MIXED_ABS;
@@ -1471,7 +1483,7 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
     // two particles per thread as on the resident path, the boundary particles after the fluid
     // (their order, the ranks it takes and its tile counts go where the resident lists, which this
     // call replaces, keep theirs); rates of boundary rows and the wall sums take the other path
-    if (nl && n >= TWIN_MIN_PARTICLES && !c->opt_wall_rates && !rhop_sum && !w_sum) {
+    if (nl && n >= TWIN_MIN_PARTICLES && twin_room(c) && !c->opt_wall_rates && !rhop_sum && !w_sum) {
         dl.order = c->perm;
         dl.rank = reinterpret_cast<const int*>(c->p1.self);
         k.threads = 64;
