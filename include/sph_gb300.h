@@ -52,8 +52,9 @@ typedef enum sph_status {
 #define SPH_FLAG_OUT_OF_GRID   0x1u  /* a particle hashed outside the grid; its cell index was clamped */
 #define SPH_FLAG_KEY_RANGE     0x2u  /* a sort key was outside [0, 2^key_bits) */
 #define SPH_FLAG_NONFINITE     0x4u  /* a non-finite position was seen by the hash kernel */
-#define SPH_FLAG_NEIGHBOR_OVERFLOW 0x8u  /* a particle had more neighbours than the list holds;
-                                            it walked its cells instead (results unaffected) */
+#define SPH_FLAG_NEIGHBOR_OVERFLOW 0x8u  /* a particle had more neighbours than list slots;
+                                            where its list is not whole it walks its cells instead
+                                            (results unaffected) */
 
 /* EOS selector: the reference hard-codes the linear form p = cs^2 (rho - rho0)
  * (src/sph/sph_run.cu:467,515); TAIT is p = B((rho/rho0)^gamma - 1), B = rho0 cs^2/gamma. */
@@ -269,8 +270,10 @@ typedef struct sph_ctx sph_ctx;
 #define SPH_OPT_PARTICLES_PER_THREAD 10  /* particles each thread of the neighbour kernels
                                     handles, grid-stride (1..64, default 1).  At the default,
                                     FP32 and SPH_PREC_MIXED_ABS runs of 400,000 particles and more
-                                    with a neighbour list, one pass-1 lane and one rebuild decision
-                                    share each list and thread between two particles (same bits) */
+                                    with a neighbour list that most particles fit, one pass-1 lane
+                                    and one rebuild decision share each list and thread between
+                                    two particles (same bits); sph_ns does so too, and otherwise
+                                    runs one particle per thread */
 /* 11 is not used (it selected a two-particles-per-thread mode, measured slower and removed) */
 #define SPH_OPT_ADAPTIVE_SKIN 13  /* 1 (default): each list rebuild picks the skin of the next
                              lists, between 0.02 and SPH_OPT_SKIN_PERMILLE, from how long the
@@ -280,9 +283,10 @@ typedef struct sph_ctx sph_ctx;
                              wall extrapolation and velocity divergence): 1 (one thread per
                              particle), 2, 4, 8 or 16 (a group of lanes shares a particle's list
                              and reduces its sums); 0 (default): 2 in FP32 with a list skin
-                             on cells of the list cutoff (SPH_OPT_CELL_DIVISIONS 1), else 1.  With groups the lists store their entries interleaved in
-                             windows of eight (a change rebuilds them).  Pass 2 runs one lane
-                             per particle (groups were slower there at every size measured) */
+                             on cells of the list cutoff (SPH_OPT_CELL_DIVISIONS 1), else 1.
+                             With groups the lists store their entries interleaved in windows of
+                             eight (a change rebuilds them).  Pass 2 runs one lane per particle
+                             (groups were slower there at every size measured) */
 #define SPH_OPT_PASS1_LANES 14  /* the same as SPH_OPT_LANES_PER_PARTICLE */
 /* 15 is not used (it selected lane groups in pass 2, removed) */
 #define SPH_OPT_CELL_DIVISIONS 16  /* cells per list cutoff of the resident grid: 1 (cells

@@ -1483,7 +1483,8 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
     // two particles per thread as on the resident path, the boundary particles after the fluid
     // (their order, the ranks it takes and its tile counts go where the resident lists, which this
     // call replaces, keep theirs); rates of boundary rows and the wall sums take the other path
-    if (nl && n >= TWIN_MIN_PARTICLES && twin_room(c) && !c->opt_wall_rates && !rhop_sum && !w_sum) {
+    if (nl && n >= TWIN_MIN_PARTICLES && twin_room(c) && c->opt_ppt == 1 && !c->opt_wall_rates &&
+        !rhop_sum && !w_sum) {
         dl.order = c->perm;
         dl.rank = reinterpret_cast<const int*>(c->p1.self);
         k.threads = 64;
