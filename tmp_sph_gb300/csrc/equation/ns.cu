@@ -367,11 +367,11 @@ k_pass2(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (GS) {
         for (int i = i0; i < k.n; i += gridDim.x * blockDim.x)
-            pass2_one<P, MODE, LIST, false>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
-                                     out_hash, err, box, disp);
+            pass2_one<P, MODE, LIST, false>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates,
+                                            out, out_hash, err, box, disp);
     } else if (i0 < k.n) {
-        pass2_one<P, MODE, LIST, false>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
-                                 out_hash, err, box, disp);
+        pass2_one<P, MODE, LIST, false>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates,
+                                        out, out_hash, err, box, disp);
     }
     if (MODE == MODE_RATES || disp == nullptr) return;
     // the block's displacement box; blockDim is a multiple of 32, every thread gets here
@@ -383,9 +383,9 @@ k_pass2(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
 // The same kernel held to CAP registers (one particle per thread): room for a chunk's four records
 // in flight with the most warps that leaves.  At 133,968 particles (linear EOS) 80 registers run
 // in 29 us, 64 in 35, 48 in 49, against 44 for one gather at a time in 40; at 380,000 80 run in
-// 45 us, 96 in 55.  More than 100 registers: the deep form (visit_fluid).  The kernel on cell-local offsets keeps 72 (380,000 particles: 77 us, 79 at 80,
-// 83 at 64).
-template <class P, int MODE, int LIST, bool GS, int CAP>
+// 45 us, 96 in 55.  More than 100 registers: the deep form (visit_fluid).  The kernel on cell-local
+// offsets keeps 72 (380,000 particles: 77 us, 79 at 80, 83 at 64).
+template <class P, int MODE, int LIST, int CAP>
 __global__ void __maxnreg__(CAP)
 k_pass2_cap(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         const unsigned* __restrict__ keys, const int* __restrict__ cs, NbrList nl,
@@ -393,15 +393,10 @@ k_pass2_cap(KParamsT<typename P::T> k, ParticleSetT<typename P::T> in,
         int wall_rates, ParticleSetT<typename P::T> out, unsigned* __restrict__ out_hash,
         unsigned* err, unsigned* disp) {
     DispBox box;
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if constexpr (GS) {
-        for (int i = i0; i < k.n; i += gridDim.x * blockDim.x)
-            pass2_one<P, MODE, LIST, (CAP > 100)>(k, i, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
-                                     out_hash, err, box, disp);
-    } else if (i0 < k.n) {
-        pass2_one<P, MODE, LIST, (CAP > 100)>(k, i0, in, keys, cs, nl, p1, rho_dt, vel_dt, wall_rates, out,
-                                 out_hash, err, box, disp);
-    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < k.n)
+        pass2_one<P, MODE, LIST, (CAP > 100)>(k, t, in, keys, cs, nl, p1, rho_dt, vel_dt,
+                                              wall_rates, out, out_hash, err, box, disp);
     if (MODE == MODE_RATES || disp == nullptr) return;
     // the block's displacement box; blockDim is a multiple of 32, every thread gets here
     __shared__ unsigned s_box[6 * (NS_MAX_THREADS / 32)];
@@ -476,14 +471,14 @@ void pass2_launch_gs(const KParamsT<typename P::T>& k, const ParticleSetT<typena
         if constexpr (MODE != MODE_RATES && !GS && (P::kId == SPH_PREC_FP32 || P::kMixed)) {
             if constexpr (L == LIST_PLAIN && kPairTwo<P>) {
                 if (k.n < DEEP_MAX_PARTICLES) {
-                    k_pass2_cap<P, MODE, L, GS, 168><<<b, k.threads, 0, s>>>(
+                    k_pass2_cap<P, MODE, L, 168><<<b, k.threads, 0, s>>>(
                         k, in, keys, cs, *nl, p1, rho_dt, vel_dt, wall_rates, out, out_hash, err,
                         disp);
                     return;
                 }
             }
             constexpr int cap = P::kCodes ? 72 : 80;
-            k_pass2_cap<P, MODE, L, GS, cap><<<b, k.threads, 0, s>>>(
+            k_pass2_cap<P, MODE, L, cap><<<b, k.threads, 0, s>>>(
                 k, in, keys, cs, *nl, p1, rho_dt, vel_dt, wall_rates, out, out_hash, err, disp);
         } else {
             k_pass2<P, MODE, L, GS><<<b, k.threads, 0, s>>>(k, in, keys, cs, *nl, p1, rho_dt,

@@ -1,6 +1,6 @@
-// ns_pair.cuh — pair arithmetic and per-particle accumulators of the two neighbour passes,
-// shared by the one-thread-per-particle kernels (ns.cu) and the lane-group kernels
-// (ns_groups.cu).  Internal to those two translation units: everything is in an unnamed
+// ns_pair.cuh — pair arithmetic and per-particle accumulators of the two neighbour passes, shared by
+// the kernels with one particle per thread (ns.cu), lane groups (ns_groups.cu) and two particles per
+// thread (ns_twin.cu).  Internal to those three translation units: everything is in an unnamed
 // namespace, so each gets its own copy.  The kernel algebra and the record layout are
 // described at the top of ns.cu.
 #pragma once

@@ -359,8 +359,8 @@ k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __rest
     // A particle overflows when its own neighbours do: counted only when the shared list is longer than
     // one particle's room, from the list just written where it is whole (a third of the candidates of
     // another walk), else from the candidates.  Only a list that is not whole sends its particles to
-    // their cells: a whole one has both, overflowed or not (765,828 particles with 80 slots, of which a
-    // few have more, 0.88 ms a step when those walked, 0.30 now; 0.33 with one particle per thread).
+    // their cells: a whole one has both, overflowed or not (765,828 disordered particles with 96 slots,
+    // which many overflow: a step 0.67 ms when those walked, 0.51 now).
     bool over = false;
     if (w.cnt > nl.cap) {
         int na = 0, nb = 0;

@@ -245,9 +245,6 @@ cudaError_t launch_pass2_rates_twin(const KParams& k, const ParticleSet& in, con
                                     float* rho_dt, float* vel_dt, cudaStream_t s);
 
 // Resident-state glue (lib/mesh.cu), one instantiation per precision policy P.
-// perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
-// cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).
-// with_tmp: also the predictor's saved state; dense: also dst.xyz.
 // The work order of the list kernels (NbrList::order) of a cell-sorted set on `grid`: its fluid
 // slots, then the others, each in slot order or (rows) with pairs of rows merged so that
 // consecutive positions hold particles one above the other.  Also fills rank (n + 1 ints: the fluid
@@ -255,6 +252,9 @@ cudaError_t launch_pass2_rates_twin(const KParams& k, const ParticleSet& in, con
 cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int* type,
                               const unsigned* keys, const int* cs, int* rank, unsigned* tiles,
                               int* order, cudaStream_t s, const unsigned* gate);
+// perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
+// cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).
+// with_tmp: also the predictor's saved state; dense: also dst.xyz.
 template <class P>
 cudaError_t launch_gather(const KParamsT<typename P::T>& k, const int* perm,
                           const ParticleSetT<typename P::T>& src, ParticleSetT<typename P::T> dst,

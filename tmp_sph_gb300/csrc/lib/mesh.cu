@@ -6,7 +6,8 @@
 // recoverD/recover (src/lib/mesh.cu:162-194).
 //
 // The sort is written for this project: reduce-then-scan LSD radix with 8-bit digits,
-// 4096-key tiles (512 threads x 8 keys), warp-level stable ranking with votes, tile-local reordering in shared memory so the scatter to global memory is in digit runs.
+// 4096-key tiles (512 threads x 8 keys), warp-level stable ranking with votes, tile-local
+// reordering in shared memory so the scatter to global memory is in digit runs.
 // No spin-waits, no allocation: all scratch is caller-provided.
 #include <cuda_runtime.h>
 
@@ -385,10 +386,11 @@ k_cell_fill(int* __restrict__ cs, int num_cells, const unsigned* __restrict__ ke
 }
 
 // Dense cell starts of a fine grid in one kernel: a block finds the slots of its CS_CELLS cells,
-// marks their first slots in shared memory and writes the cells out, each once.  The general path (clear, mark, fill) writes every cell twice and reads it once, and its
-// one-thread searches took 22 dependent loads a block.  4.96M particles on 50M cells: 0.31 ms there,
-// 0.09 here.  A block walks all slots of its cells, so this is for grids with more cells than
-// particles; coarse cells hold tens of thousands of slots per CS_CELLS.
+// marks their first slots in shared memory and writes the cells out, each once.  The general path
+// (clear, mark, fill) writes every cell twice and reads it once, and its one-thread searches took 22
+// dependent loads a block.  4.96M particles on 50M cells: 0.31 ms there, 0.09 here.  A block walks all
+// slots of its cells, so this is for grids with more cells than particles; coarse cells hold tens of
+// thousands of slots per CS_CELLS.
 constexpr int CS_THREADS = 256;
 constexpr int CS_WARPS = CS_THREADS / 32;
 constexpr int CS_CELLS = 4096;
