@@ -13,10 +13,10 @@ pytestmark = pytest.mark.gpu
 KEYS = ("pos", "vel", "rho", "p")
 
 
-def with_fluid(pos, dx, seed=0):
-    """The empty 1.0 x 0.5 x 0.6 m tank with fluid particles at `pos`, moving at random."""
+def with_fluid(pos, dx, seed=0, tank=(1.0, 0.5, 0.6)):
+    """The empty tank with fluid particles at `pos`, moving at random."""
     from tmp_sph_gb300 import cases
-    st, p = cases.build("small", physics="config", dx=dx, block=(0.2, 0.2, 0.1))
+    st, p = cases.build("small", physics="config", dx=dx, tank=tank, block=(0.2, 0.2, 0.1))
     wall = st["type"] != 1
     m = len(pos)
     vel = np.random.default_rng(seed).uniform(-0.5, 0.5, (m, 3))
@@ -92,6 +92,39 @@ def test_instances_stay_apart(sphlib, cuda, kind, precision):
         ref = run(st, p, {api.SPH_OPT_SKIN_PERMILLE: 0}, precision, steps=2)
         for k in KEYS:
             assert np.array_equal(out[k][off[b]:off[b + 1]], ref[k]), (b, k)
+
+
+def test_many_small_instances(sphlib, cuda):
+    """700 tanks of 0.2 m: more than 1024 runs of one instance and kind in the work order."""
+    from tmp_sph_gb300 import api
+    made = [with_fluid(np.array([-0.33, -0.13, -0.2]) + drop(b, 0.04), 0.04, seed=b,
+                       tank=(0.2, 0.2, 0.2)) for b in range(700)]
+    states, p = [m[0] for m in made], made[0][1]
+    assert sum(len(s["rho"]) for s in states) >= 400000
+    out, off = run_batch(states, p, {api.SPH_OPT_SKIN_PERMILLE: 0}, "fp32")
+    for b in [0, 1, 2, 3, 321, 322, 323, 324, 400, 510, 511, 512, 513, 697, 698, 699]:
+        ref = run(states[b], p, {api.SPH_OPT_SKIN_PERMILLE: 0}, "fp32", steps=2)
+        for k in KEYS:
+            assert np.array_equal(out[k][off[b]:off[b + 1]], ref[k]), (b, k)
+
+
+def test_particles_outside_the_search(sphlib, cuda):
+    """Escaped particles outside the search (park_inactive) come after all instances: each instance
+    as alone, whatever their number."""
+    from tmp_sph_gb300 import api
+    states, p = batch_of(film)
+    for b, st in enumerate(states):  # an odd or even number of them above the tank's rim
+        up = np.arange(5 + b % 3)
+        st["pos"][up] = np.array([0.3, 0.2, 0.66]) + 0.005 * up[:, None].astype(np.float32)
+    p.park_inactive = 1
+    out, off = run_batch(states, p, {api.SPH_OPT_SKIN_PERMILLE: 0}, "fp32")
+    parked = 0
+    for b, st in enumerate(states):
+        ref = run(st, p, {api.SPH_OPT_SKIN_PERMILLE: 0}, "fp32", steps=2)
+        parked += int(np.all(ref["pos"][:8] == np.array(p.escape_park, np.float32), axis=1).sum())
+        for k in KEYS:
+            assert np.array_equal(out[k][off[b]:off[b + 1]], ref[k]), (b, k)
+    assert parked == sum(5 + b % 3 for b in range(len(states)))
 
 
 @pytest.mark.parametrize("kind,opts", [(drop, {}), (heavy_drop, {"SPH_OPT_NEIGHBOR_CAP": 96}),

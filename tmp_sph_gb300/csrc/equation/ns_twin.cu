@@ -23,8 +23,11 @@
 // lists prefetched into L2 ahead of their use (level).
 //
 // The two particles must be of one simulation: candidates are told apart by distance alone, and
-// batched instances hold positions in a frame of their own each.  A thread on the seam of two
-// instances (at most two per instance) keeps a list of each particle in its half of the column.
+// batched instances hold positions in a frame of their own each.  The work order of a batch gives each
+// instance's fluid and each one's walls an even number of positions, so no thread holds two instances.
+// (A list of each particle in its half of the column, for the threads on a seam, kept the pairs but not
+// the time: such a thread reads two lists one after the other, and its warp waits.  16 tanks of 25,000
+// particles 0.22 ms a step, 0.15 with even positions.)
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -36,33 +39,32 @@ namespace sph {
 
 namespace {
 
-// The two particles of thread u: slots a and b (b = a when u has one particle only).
+// The two particles of thread u: slots a and b (b = a when u has one particle only).  BATCH: of a padded
+// work order, where no slot is -1 (none of a thread past the last instance).
 struct Twin {
     int a, b;
     bool two;
 };
+template <bool BATCH>
 __device__ __forceinline__ Twin twin_of(const NbrList& nl, int u, int n) {
     Twin w;
     w.a = work_slot(nl, 2 * u);
-    w.two = 2 * u + 1 < n;
-    w.b = w.two ? work_slot(nl, 2 * u + 1) : w.a;
+    if constexpr (BATCH) {
+        const int b = work_slot(nl, 2 * u + 1);
+        w.two = b >= 0;
+        w.b = w.two ? b : w.a;
+    } else {
+        w.two = 2 * u + 1 < n;
+        w.b = w.two ? work_slot(nl, 2 * u + 1) : w.a;
+    }
     return w;
 }
 // Column of thread u's list: as nbr_col, with the slots of its two particles.
 __device__ __forceinline__ size_t twin_col(const NbrList& nl, int u) {
     return (size_t)(u >> 5) * ((size_t)nl.cap << 6) + ((size_t)(u & 31) << 2);
 }
-// nl.count of a thread: the entries of its shared list; TWIN_WALKS when they do not fit it; below that,
-// of two instances, the chunks of its particles' own lists (split_count).
+// nl.count of a thread: the entries of its shared list, TWIN_WALKS when they do not fit it.
 constexpr int TWIN_WALKS = -1;
-constexpr int SPLIT_BITS = 15;
-__device__ __forceinline__ int split_count(int chunks_a, int chunks_b) {
-    return TWIN_WALKS - 1 - (chunks_a << SPLIT_BITS | chunks_b);
-}
-__device__ __forceinline__ int split_chunks(int cnt, int m) {
-    const int c = TWIN_WALKS - 1 - cnt;
-    return m ? c & ((1 << SPLIT_BITS) - 1) : c >> SPLIT_BITS;
-}
 
 // ---------------------------------------------------------------- list build
 // One particle's side of the build: its cell and the part of a strip its cutoff sphere reaches.
@@ -130,64 +132,17 @@ struct RingWriter {
     }
 };
 
-// The own lists of two particles of different instances, as k_nbr_build makes them: a particle's
-// entries in its half of the column, walk order, itself left out.  A call, not inlined: few threads
-// take it, and inlined it made the build spill.
-template <class P>
-__device__ __noinline__ void build_split(const KParamsT<float>& k, const NbrList& nl,
-                                         const float4* __restrict__ X,
-                                         const unsigned* __restrict__ keys,
-                                         const int* __restrict__ cs, int u, int* ring,
-                                         unsigned* err) {
-    const float cut2 = nl.cut2 ? __ldg(nl.cut2) : k.kh2_list;
-    const Twin tw = twin_of(nl, u, k.n);
-    int chunks[2], most = 0;
-#pragma unroll 1
-    for (int m = 0; m < 2; m++) {
-        const int i = m ? tw.b : tw.a;
-        const float4 pi = X[i];
-        const TwinWalk w = twin_walk<P>(k, pi, keys[i], cut2);
-        const bool all = fluid_rec(pi.w);
-        RingWriter out(nl.idx + twin_col(nl, u) + (m ? (size_t)nl.cap << 5 : 0), nl.cap, ring);
-#pragma unroll 1
-        for (int z = max(w.cz - k.reach, 0); z <= min(w.cz + k.reach, k.gz - 1); z++) {
-#pragma unroll 1
-            for (int y = max(w.cy - k.reach, 0); y <= min(w.cy + k.reach, k.gy - 1); y++) {
-                int xl, xh;
-                if (!w.strip(k, y, z, xl, xh)) continue;
-                const int row = (z * k.gy + y) * k.gx;
-                const int j1 = min(__ldg(cs + row + xh + 1), k.n);
-                for (int j = max(__ldg(cs + row + xl), 0); j < j1; j++) {
-                    const float4 p = ld_pos(X, (size_t)j);
-                    float dx, dy, dz;
-                    rel_pos<P>(k, pi, p, 0u, dx, dy, dz);
-                    out.offer(j, j != i && (all || fluid_rec(p.w)) && dist2(dx, dy, dz) < cut2);
-                    out.drain();
-                }
-            }
-        }
-        out.flush(pad_slot<P>(k.n));
-        chunks[m] = (out.cnt + 3) >> 2;
-        most = max(most, out.cnt);
-    }
-    const bool over = most > nl.cap;
-    nl.count[u] = over || (most + 3) >> 2 >= 1 << SPLIT_BITS ? TWIN_WALKS
-                                                             : split_count(chunks[0], chunks[1]);
-    raise_flags(err, over ? SPH_FLAG_NEIGHBOR_OVERFLOW : 0u);
-}
-
 // The shared lists.  Bound by instructions (62% issue, 40% of the ALU pipe; about 390 candidates a
 // warp for 100 listed slots).  4.96M particles, 1.60 ms with a window per particle and strip and a
 // branch per candidate; 1.27 with one walk over the rows and cells either sphere reaches; 1.16 with
 // branch-free candidates on top; 1.05 with near_fluid on the fluid ranks.
 //
-// BATCH: batched instances, whose seams build_split takes.
+// BATCH: batched instances, on a padded work order (twin_of).
 template <class P, bool BATCH>
 __global__ void __launch_bounds__(TWIN_BUILD_THREADS)
-k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __restrict__ X,
-                 const unsigned* __restrict__ keys, const int* __restrict__ cs,
-                 const __grid_constant__ NbrList nl, float4* rec, float4* nrec, unsigned* err,
-                 const unsigned* gate) {
+k_nbr_build_twin(KParamsT<float> k, const float4* __restrict__ X,
+                 const unsigned* __restrict__ keys, const int* __restrict__ cs, NbrList nl,
+                 float4* rec, float4* nrec, unsigned* err, const unsigned* gate) {
     __shared__ int s_ring[RingWriter::RING * TWIN_BUILD_THREADS];
     if (gated_off(gate)) return;
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
@@ -195,9 +150,10 @@ k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __rest
         pad_record<float>(rec, k.n);
         pad_record<float>(nrec, k.n);
     }
-    if (2 * u >= k.n) return;
+    if (2 * u >= (BATCH ? k.positions : k.n)) return;
     const float cut2 = nl.cut2 ? __ldg(nl.cut2) : k.kh2_list;
-    const Twin tw = twin_of(nl, u, k.n);
+    const Twin tw = twin_of<BATCH>(nl, u, k.n);
+    if (BATCH && tw.a < 0) return;
     const int a = tw.a, b = tw.b;
     const float4 pa = X[a], pb = X[b];
     if (nl.xb) {
@@ -210,12 +166,6 @@ k_nbr_build_twin(const __grid_constant__ KParamsT<float> k, const float4* __rest
         !(wb.on && near_fluid(k, cs, nl.rank, wb.cx, wb.cy, wb.cz))) {
         nl.count[u] = 0;
         return;
-    }
-    if constexpr (BATCH) {
-        if (keys[a] / (unsigned)k.inst_cells != keys[b] / (unsigned)k.inst_cells) {
-            build_split<P>(k, nl, X, keys, cs, u, s_ring, err);
-            return;
-        }
     }
     const int r = k.reach;
     // two particles next to each other in one layer, each inside its cell
@@ -404,30 +354,9 @@ __device__ __forceinline__ void visit_twin(const NbrList& nl, const float4* __re
     });
 }
 
-// The pairs of particle m (0 or 1) of a thread of two instances, from its own list: one(j, a, v, dx,
-// dy, dz, r2) inside the support radius.
-template <class P, class F>
-__device__ __forceinline__ void visit_split(const KParamsT<float>& k, const NbrList& nl,
-                                            const float4* __restrict__ R, int u, int m, int cnt,
-                                            const float4& pi, F&& one) {
-    for_each_chunk<false>(nl.idx + twin_col(nl, u) + (m ? (size_t)nl.cap << 5 : 0),
-                          split_chunks(cnt, m) << 2, 0, 1, [&](const int4& q) {
-        const int e[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            float4 a, v;
-            ld_rec(R, e[c], a, v);
-            float dx, dy, dz;
-            rel_pos<P>(k, pi, a, 0u, dx, dy, dz);
-            const float r2 = dist2(dx, dy, dz);
-            if (r2 < k.kh2) one(e[c], a, v, dx, dy, dz, r2);
-        }
-    });
-}
-
 // The cells of two particles that do not fit their list, when they are of one cell or of neighbouring
 // ones: one box of cells holds the walks of both, and a candidate that only one of them walks lies
-// outside the other's support radius.  (Never two instances: empty layers lie between their cells.)
+// outside the other's support radius.
 struct TwinCells {
     int xl, xh, yl, yh, zl, zh;
     bool near;
@@ -528,16 +457,14 @@ __device__ __forceinline__ void pass2_twin(const KParamsT<float>& k, Pass2Acc<P,
     add_if(r2b, k.kh2, wb, eb, cb, bx, by, bz, B.sd.s, B.sx.s, B.sy.s, B.sz.s);
 }
 
-// BATCH: batched instances, whose threads on a seam read two lists (visit_split).  The branch moves
-// registers about, so one simulation runs without it: ten steps of a surge of 765,828 particles 4.02
-// ms, 4.07 with it.
 template <class P, bool BATCH>
 __global__ void __maxnreg__(80)
 k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ keys,
              const int* __restrict__ cs, NbrList nl, Pass1Out out) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (2 * u >= k.n) return;
-    const Twin tw = twin_of(nl, u, k.n);
+    if (2 * u >= (BATCH ? k.positions : k.n)) return;
+    const Twin tw = twin_of<BATCH>(nl, u, k.n);
+    if (BATCH && tw.a < 0) return;
     Pass1Acc<P> A, B;
     A.load(in.rec, tw.a);
     B.load(in.rec, tw.b);
@@ -571,20 +498,13 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
 #pragma unroll 1
             for (int m = 0; m < 2; m++) {
                 Pass1Acc<P> C = m ? B : A;
-                if (BATCH && cnt < TWIN_WALKS)
-                    visit_split<P>(k, nl, in.rec, u, m, cnt, C.pi,
-                                   [&](int, const float4& aj, const float4& vj, float dx, float dy,
-                                       float dz, float r2) {
-                        C.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
-                    });
-                else
-                    walk_pairs<P, 2>(k, cs, keys, in.rec, m ? tw.b : tw.a, C.pi, k.kh2,
-                                     [&](int j, unsigned, const float4&, float dx, float dy,
-                                         float dz, float r2) {
-                        float4 aj, vj;
-                        ld_rec(in.rec, j, aj, vj);
-                        C.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
-                    });
+                walk_pairs<P, 2>(k, cs, keys, in.rec, m ? tw.b : tw.a, C.pi, k.kh2,
+                                 [&](int j, unsigned, const float4&, float dx, float dy, float dz,
+                                     float r2) {
+                    float4 aj, vj;
+                    ld_rec(in.rec, j, aj, vj);
+                    C.pair(k, aj, vj, dx, dy, dz, r2, 0.f);
+                });
                 if (m) B = C;
                 else A = C;
             }
@@ -594,6 +514,8 @@ k_pass1_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
     if (tw.two) B.template finish<false>(k, out, nullptr, nullptr, tw.b);
 }
 
+// The caps leave both at ten blocks of 64 per SM: 96 registers of 104, in a batch 94 of 96 (96 of 104
+// there cost six dam breaks of 5.0M particles 0.8% of their steps).
 template <class P, int MODE, bool BATCH>
 __global__ void __maxnreg__(BATCH ? 96 : 104)
 k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ keys,
@@ -602,8 +524,8 @@ k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
              unsigned* err, unsigned* disp) {
     DispBox box;
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (2 * u < k.n) {
-        const Twin tw = twin_of(nl, u, k.n);
+    if (2 * u < (BATCH ? k.positions : k.n) && (!BATCH || work_slot(nl, 2 * u) >= 0)) {
+        const Twin tw = twin_of<BATCH>(nl, u, k.n);
         Pass2Acc<P, MODE> A, B;
         A.load(k, p1, tw.a, 0);
         B.load(k, p1, tw.b, 0);
@@ -623,13 +545,7 @@ k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
 #pragma unroll 1
                     for (int m = 0; m < 2; m++) {
                         Pass2Acc<P, MODE> C = m ? B : A;
-                        if (BATCH && C.active && cnt < TWIN_WALKS)
-                            visit_split<P>(k, nl, p1.nrec, u, m, cnt, C.pi,
-                                           [&](int j, const float4& aj, const float4& vj, float dx,
-                                               float dy, float dz, float r2) {
-                                C.pair(k, p1, j, aj, vj, dx, dy, dz, r2, 0.f);
-                            });
-                        else if (C.active)
+                        if (C.active)
                             walk_pairs<P, 2>(k, cs, keys, p1.nrec, m ? tw.b : tw.a, C.pi, k.kh2,
                                              [&](int j, unsigned, const float4&, float dx, float dy,
                                                  float dz, float r2) {
@@ -656,7 +572,9 @@ k_pass2_twin(KParamsT<float> k, ParticleSet in, const unsigned* __restrict__ key
     reduce_disp_box(box, disp, s_box);
 }
 
-inline int twin_blocks(int n, int threads) { return (n + 2 * threads - 1) / (2 * threads); }
+inline int twin_blocks(int positions, int threads) {
+    return (positions + 2 * threads - 1) / (2 * threads);
+}
 
 }  // namespace
 
@@ -665,7 +583,7 @@ cudaError_t launch_nbr_build_twin(const KParams& k, const ParticleSet& in, const
                                   const int* cs, const NbrList& nl, float4* nrec, unsigned* err,
                                   cudaStream_t s, const unsigned* gate) {
     if (k.n <= 0) return cudaSuccess;
-    const int blocks = twin_blocks(k.n, TWIN_BUILD_THREADS);
+    const int blocks = twin_blocks(k.positions, TWIN_BUILD_THREADS);
     if (k.inst_cells)
         k_nbr_build_twin<P, true><<<blocks, TWIN_BUILD_THREADS, 0, s>>>(k, in.xyz, keys, cs, nl,
                                                                          in.rec, nrec, err, gate);
@@ -680,7 +598,7 @@ cudaError_t launch_pass1_twin(const KParams& k, const ParticleSet& in, const uns
                               const int* cs, const NbrList& nl, const Pass1Out& out,
                               cudaStream_t s) {
     if (k.n <= 0) return cudaSuccess;
-    const int blocks = twin_blocks(k.n, k.threads);
+    const int blocks = twin_blocks(k.positions, k.threads);
     if (k.inst_cells)
         k_pass1_twin<P, true><<<blocks, k.threads, 0, s>>>(k, in, keys, cs, nl, out);
     else
@@ -694,7 +612,7 @@ cudaError_t launch_pass2_twin(const KParams& k, HalfStep half, const ParticleSet
                               const Pass1Out& p1, ParticleSet out, unsigned* out_hash,
                               unsigned* err, unsigned* disp, cudaStream_t s) {
     if (k.n <= 0) return cudaSuccess;
-    const int blocks = twin_blocks(k.n, k.threads);
+    const int blocks = twin_blocks(k.positions, k.threads);
     auto launch = [&](auto mode, auto batch) {
         k_pass2_twin<P, decltype(mode)::value, decltype(batch)::value>
             <<<blocks, k.threads, 0, s>>>(k, in, keys, cs, nl, p1, nullptr, nullptr, out, out_hash,
@@ -713,7 +631,7 @@ cudaError_t launch_pass2_rates_twin(const KParams& k, const ParticleSet& in, con
                                     const int* cs, const NbrList& nl, const Pass1Out& p1,
                                     float* rho_dt, float* vel_dt, cudaStream_t s) {
     if (k.n <= 0) return cudaSuccess;
-    k_pass2_twin<PrecF32, MODE_RATES, false><<<twin_blocks(k.n, k.threads), k.threads, 0, s>>>(
+    k_pass2_twin<PrecF32, MODE_RATES, false><<<twin_blocks(k.positions, k.threads), k.threads, 0, s>>>(
         k, in, keys, cs, nl, p1, rho_dt, vel_dt, ParticleSet{}, nullptr, nullptr, nullptr);
     return cudaGetLastError();
 }

@@ -95,6 +95,9 @@ struct KParamsT {
     // (unused by the FP64 kernels)
     unsigned long long inv_h2, m_half_inv_h2, one2, m_half2, c_fr2, c_fr_mass2, eta2_2,
         delta_h_cs2, visc2;
+    // work positions of the list kernels: n, or more where a batch's order is padded
+    // (launch_work_order).  Last: moving the members above cost the shared-list passes 1.5%
+    int positions;
 };
 using KParams = KParamsT<float>;
 

@@ -177,8 +177,8 @@ struct NbrList {
     // every particle is rebuilt at cut2
     const unsigned* iw = nullptr;
     const int* inst = nullptr;
-    // work order: thread t of the list kernels takes slot order[t] (all fluid slots first), and
-    // the list columns and counts are indexed by t; NULL: slot t
+    // work order: thread t of the list kernels takes slot order[t] (all fluid slots first; none at
+    // -1, in a padded order), and the list columns and counts are indexed by t; NULL: slot t
     const int* order = nullptr;
 };
 // Particles of a lattice of spacing dx within kh (1 + skin) of a point.
@@ -248,10 +248,14 @@ cudaError_t launch_pass2_rates_twin(const KParams& k, const ParticleSet& in, con
 // The work order of the list kernels (NbrList::order) of a cell-sorted set on `grid`: its fluid
 // slots, then the others, each in slot order or (rows) with pairs of rows merged so that
 // consecutive positions hold particles one above the other.  Also fills rank (n + 1 ints: the fluid
-// slots before each slot).  Scratch: tiles (one word per 4096 slots).
-cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int* type,
-                              const unsigned* keys, const int* cs, int* rank, unsigned* tiles,
-                              int* order, cudaStream_t s, const unsigned* gate);
+// slots before each slot).  Scratch: tiles (one word per 4096 slots, and padding_for(n_inst)).
+// n_inst > 0 pads the order of n_inst batched instances of inst_cells cells each to an even number of
+// positions per instance and kind, -1 where there is no slot: order has n + padding_for(n_inst)
+// entries.
+constexpr int padding_for(int n_inst) { return 2 * (n_inst + 1); }
+cudaError_t launch_work_order(int n, const sph_params& grid, int rows, int n_inst, int inst_cells,
+                              const int* type, const unsigned* keys, const int* cs, int* rank,
+                              unsigned* tiles, int* order, cudaStream_t s, const unsigned* gate);
 // perm == NULL copies slot for slot.  With cell codes a permuting gather recomputes the
 // cell-local offsets from the FP64 positions for the cells in `keys` (the new sorted keys).
 // with_tmp: also the predictor's saved state; dense: also dst.xyz.

@@ -645,12 +645,63 @@ k_fluid_rank(int n, const int* __restrict__ type, const unsigned* __restrict__ t
     }
 }
 
+// First positions of the fluid of every instance and then of the walls of every instance (first[0 ..
+// n_inst] and first[n_inst + 1 ..]; instance n_inst: the slots outside the neighbour search) in an order
+// that gives each of them an even number of positions, and -1 at the positions without a slot.  One
+// block.  The slots of instance b start at those of its first cell.
+__global__ void __launch_bounds__(1024)
+k_work_segments(int n, int n_inst, int inst_cells, const int* __restrict__ cs,
+                const int* __restrict__ rank, int* __restrict__ first, int* __restrict__ order,
+                const unsigned* gate) {
+    __shared__ int s_w[32];
+    if (gated_off(gate)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int segments = 2 * (n_inst + 1), limit = n + segments;
+    int carry = 0;
+    for (int base = 0; base < segments; base += 1024) {
+        const int q = base + tid;
+        int count = 0;
+        if (q < segments) {
+            const bool fluid = q <= n_inst;
+            const int b = fluid ? q : q - n_inst - 1;
+            const int s = min(max(cs[(size_t)b * inst_cells], 0), n);
+            const int e = b < n_inst ? min(max(cs[(size_t)(b + 1) * inst_cells], s), n) : n;
+            const int f = rank[e] - rank[s];
+            count = fluid ? f : e - s - f;
+        }
+        const int room = (count + 1) & ~1;
+        int incl = room;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_w[warp] = incl;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 32; w++) {
+            if (w < warp) before += s_w[w];
+            all += s_w[w];
+        }
+        const int at = carry + before + incl - room;
+        if (q < segments) {
+            first[q] = at;
+            if (room > count && (unsigned)(at + count) < (unsigned)limit) order[at + count] = -1;
+        }
+        carry += all;
+        __syncthreads();
+    }
+    for (int t = carry + tid; t < limit; t += 1024) order[t] = -1;
+}
+
 // order[position of slot i] = i.  The fluid slots come first, then the others, each in slot order
 // or, with `rows`, with the rows y = 2m and 2m + 1 of a layer merged by cell x (a particle of the
 // even row before one of the odd row): consecutive positions then hold particles one above the
 // other.  The merged position is the rank in the own row plus the partner row's particles before
-// it, both from the dense cell starts.
-__global__ void k_work_order(int n, int gx, int gy, unsigned num_cells, int rows,
+// it, both from the dense cell starts.  With `first` (k_work_segments; instances of inst_cells cells)
+// each instance's slots of a kind start there.
+__global__ void k_work_order(int n, int gx, int gy, unsigned num_cells, int rows, int n_inst,
+                             int inst_cells, const int* __restrict__ first,
                              const int* __restrict__ type, const int* __restrict__ rank,
                              const unsigned* __restrict__ keys, const int* __restrict__ cs,
                              int* __restrict__ order, const unsigned* gate) {
@@ -678,8 +729,16 @@ __global__ void k_work_order(int n, int gx, int gy, unsigned num_cells, int rows
             pos += odd ? ahead - (start(own) - start(other)) : ahead;
         }
     }
-    if (!fluid) pos += nf;
-    if ((unsigned)pos < (unsigned)n) order[pos] = i;
+    int limit = n;
+    if (first) {
+        const int b = min((int)(key / (unsigned)inst_cells), n_inst);
+        const int s = min(max(__ldg(cs + (size_t)b * inst_cells), 0), n);
+        pos += __ldg(first + (fluid ? b : n_inst + 1 + b)) - before(s);
+        limit += padding_for(n_inst);
+    } else if (!fluid) {
+        pos += nf;
+    }
+    if ((unsigned)pos < (unsigned)limit) order[pos] = i;
 }
 
 // Instance of particle i when instance b owns [off[b], off[b+1]) (upper bound search).
@@ -1012,17 +1071,23 @@ cudaError_t build_cell_starts(const unsigned* sorted_keys, int n, int num_cells,
     return cudaGetLastError();
 }
 
-cudaError_t launch_work_order(int n, const sph_params& grid, int rows, const int* type,
-                              const unsigned* keys, const int* cs, int* rank, unsigned* tiles,
-                              int* order, cudaStream_t s, const unsigned* gate) {
+cudaError_t launch_work_order(int n, const sph_params& grid, int rows, int n_inst, int inst_cells,
+                              const int* type, const unsigned* keys, const int* cs, int* rank,
+                              unsigned* tiles, int* order, cudaStream_t s, const unsigned* gate) {
     if (n <= 0) return cudaSuccess;
     const int nt = blocks_for((long)n + 1, WO_TILE);
     k_fluid_count<<<nt, WO_THREADS, 0, s>>>(n, type, tiles, gate);
     k_fluid_scan<<<1, 1024, 0, s>>>(nt, tiles, gate);
     k_fluid_rank<<<nt, WO_THREADS, 0, s>>>(n, type, tiles, rank, gate);
+    int* first = nullptr;
+    if (n_inst > 0) {
+        first = reinterpret_cast<int*>(tiles + nt);
+        k_work_segments<<<1, 1024, 0, s>>>(n, n_inst, inst_cells, cs, rank, first, order, gate);
+    }
     k_work_order<<<blocks_for(n, 256), 256, 0, s>>>(n, grid.grid_dim[0], grid.grid_dim[1],
-                                                    (unsigned)grid.num_cells, rows, type, rank,
-                                                    keys, cs, order, gate);
+                                                    (unsigned)grid.num_cells, rows, n_inst,
+                                                    inst_cells, first, type, rank, keys, cs, order,
+                                                    gate);
     return cudaGetLastError();
 }
 

@@ -89,6 +89,7 @@ KParams make_kparams(const sph_params& p, int n) {
     k.park_z = p.escape_park[2];
     k.park_inactive = p.park_inactive;
     k.inst_boxes = 0;
+    k.positions = n;
     k.code_bias2 = two_floats(-8388609.f, -8388612.f);
     k.inv_h2 = twice(k.inv_h);
     k.m_half_inv_h2 = twice(-0.5f * k.inv_h);
@@ -167,6 +168,7 @@ KParamsT<double> make_kparams_t<double>(const sph_params& p, int n) {
     k.park_z = p.escape_park[2];
     k.park_inactive = p.park_inactive;
     k.inst_boxes = 0;
+    k.positions = n;
     return k;
 }
 

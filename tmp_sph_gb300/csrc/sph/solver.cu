@@ -316,6 +316,12 @@ static bool twin_lists(const sph_ctx* c) {
     return fp32_pairs(c->prec) && c->opt_nbr_list && pass1_lanes(c) == 1 && c->opt_ppt == 1 &&
            !per_instance(c) && c->n >= TWIN_MIN_PARTICLES && twin_room(c);
 }
+// Whether the work order is padded, so that no two instances of a batch share a list.
+static bool padded_order(const sph_ctx* c) { return c->n_inst > 1 && twin_lists(c); }
+// Room for that padding: contexts that may hold enough particles.
+static int most_padding(int capacity) {
+    return capacity >= TWIN_MIN_PARTICLES ? padding_for(SPH_MAX_INSTANCES) : 0;
+}
 template <class P>
 constexpr bool kTwin = P::kId == SPH_PREC_FP32 || P::kId == SPH_PREC_MIXED_ABS;
 
@@ -360,6 +366,7 @@ KParamsT<T> resident_kparams(const sph_ctx* c) {
     k.gz_stride = c->n_inst > 1 ? instance_stride(c->gz_inst, c->opt_reach) : c->gz_inst;
     k.inst_boxes = per_instance(c) ? 1 : 0;
     k.inst_cells = c->n_inst > 1 ? c->Pi.grid_dim[0] * c->Pi.grid_dim[1] * k.gz_stride : 0;
+    k.positions = c->n + (padded_order(c) ? padding_for(c->n_inst) : 0);
     const double cut = (double)c->P.kh * (1.0 + (c->skin > 0.0 ? c->skin : 0.0));
     k.kh2_list = (T)(cut * cut);
     if (k.kh2_list < k.kh2) k.kh2_list = k.kh2;
@@ -611,8 +618,10 @@ cudaError_t rebuild_lists(sph_ctx* c, const KParamsT<typename P::T>& k, HalfStep
         cudaSuccess)
         return e;
     // the permutation just applied, the sort's scratch and the pass-1 records hold nothing now
-    if (nl && (e = launch_work_order(c->n, c->Pi, twin_lists(c) ? 1 : 0, y.type, c->keys_sorted,
-                                     c->cell_start, reinterpret_cast<int*>(State<P>::p1(c).self),
+    if (nl && (e = launch_work_order(c->n, c->Pi, twin_lists(c) ? 1 : 0,
+                                     padded_order(c) ? c->n_inst : 0, k.inst_cells, y.type,
+                                     c->keys_sorted, c->cell_start,
+                                     reinterpret_cast<int*>(State<P>::p1(c).self),
                                      static_cast<unsigned*>(c->sort_scratch), c->perm, s,
                                      gate)) != cudaSuccess)
         return e;
@@ -762,7 +771,8 @@ cudaError_t alloc_list(sph_ctx* c) {
     if (c->nl.idx && c->nl.cap == cap) return cudaSuccess;
     free_list(c->nl);
     // warp-interleaved blocks of cap x 32 slots: whole warps, the last one padded
-    const size_t rows = ((size_t)(c->capacity > 0 ? c->capacity : 1) + 63) & ~(size_t)63;
+    const size_t most = (size_t)(c->capacity > 0 ? c->capacity : 1) + most_padding(c->capacity);
+    const size_t rows = (most + 63) & ~(size_t)63;
     cudaError_t e = dalloc(&c->nl.idx, (size_t)cap * rows);
     if (e == cudaSuccess) e = dalloc(&c->nl.count, c->capacity);
     if (e == cudaSuccess) e = dalloc(&c->nl.xb, c->capacity);
@@ -793,7 +803,7 @@ extern "C" int sph_create(const sph_params* p, int capacity, sph_ctx** out) {
     if (e == cudaSuccess) e = alloc_state(c);
     if (e == cudaSuccess) e = dalloc(&c->hash_x, cap);
     if (e == cudaSuccess) e = dalloc(&c->keys_sorted, cap);
-    if (e == cudaSuccess) e = dalloc(&c->perm, cap);
+    if (e == cudaSuccess) e = dalloc(&c->perm, (size_t)cap + most_padding(cap));
     c->cell_capacity = std::max(p->num_cells, c->Pi.num_cells);
     if (e == cudaSuccess) e = dalloc(&c->cell_start, (size_t)c->cell_capacity + 1);
     c->sort_scratch_bytes = sort_scratch_bytes(cap);
@@ -1488,7 +1498,7 @@ extern "C" int sph_ns(sph_ctx* c, float* s_pos, float* s_vel, float* s_rho, floa
         dl.order = c->perm;
         dl.rank = reinterpret_cast<const int*>(c->p1.self);
         k.threads = 64;
-        if (launch_work_order(n, c->P, 0, c->x.type, c->keys_sorted, c->cell_start,
+        if (launch_work_order(n, c->P, 0, 0, 0, c->x.type, c->keys_sorted, c->cell_start,
                               reinterpret_cast<int*>(c->p1.self),
                               static_cast<unsigned*>(c->sort_scratch), c->perm, s,
                               nullptr) != cudaSuccess ||
