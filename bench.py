@@ -63,9 +63,10 @@ PHASE_BYTES = {"sort": B_SORT, "gather_cells": B_PERMUTE, "nbr_build": 16, "pass
                "pass2_integrate": B_PASS2 + B_INTEGRATE + B_HASH}
 PHASE_KERNEL = {"sort": "k_rs_upsweep/k_rs_scan/k_rs_downsweep",
                 "gather_cells": "k_gather + k_cell_starts (k_cell_mark/k_cell_fill) + k_work_order",
-                "nbr_build": "k_nbr_build (one cell walk; positions read once = 16 B)",
-                "pass1": "k_pass1 (k_pass1_g with two or four lanes)",
-                "pass2_integrate": "k_pass2<MODE_PRED|MODE_CORR>"}
+                "nbr_build": "k_nbr_build_twin, or k_nbr_build with one particle per thread (one cell "
+                             "walk; positions read once = 16 B)",
+                "pass1": "k_pass1_twin (k_pass1; k_pass1_g with lane groups)",
+                "pass2_integrate": "k_pass2_twin<MODE_PRED|MODE_CORR> (k_pass2_cap, k_pass2)"}
 
 
 def dist_env():
@@ -183,10 +184,11 @@ def build_case(name: str):
 
 
 def count_launches(num_cells: int, half_steps: int, rebuilds: int, mode: str,
-                   keep_keys: bool = False, particles: int = 0) -> int:
+                   keep_keys: bool = False, particles: int = 0, padded: bool = False) -> int:
     """Kernels launched over `half_steps` half steps with `rebuilds` list rebuilds
-    (keep_keys: a batch with per-instance decisions, one more kernel per rebuild; particles: with
-    that many and neighbour lists, 0: the cell list and list build alone, marked and filled)."""
+    (keep_keys: a batch with per-instance decisions, padded: one with lists shared by two particles,
+    one more kernel per rebuild each; particles: with that many and neighbour lists, 0: the cell list
+    and list build alone, marked and filled)."""
     bits = 1
     while bits < 31 and (1 << bits) < num_cells:
         bits += 1
@@ -195,7 +197,7 @@ def count_launches(num_cells: int, half_steps: int, rebuilds: int, mode: str,
     # clear, 3 kernels per radix pass, gather + copy back, cell-start clear, mark and fill,
     # and the neighbour-list build.  In gated mode the rebuild kernels are launched every
     # half step (and return at once when the lists are kept).
-    rebuild_kernels = 3 * passes + 7 + (1 if keep_keys else 0)
+    rebuild_kernels = 3 * passes + 7 + (1 if keep_keys else 0) + (1 if padded else 0)
     if particles:
         # the four kernels of the work order; grids with a cell or more per particle get their
         # cell starts from one kernel instead of three
@@ -583,6 +585,10 @@ def batch_measure(n_inst: int, precision: str, args, stream, steps: int, warmup:
     ms = replicas.reduce_max(ev0.elapsed_time(ev1))
     rebuilds = sol.rebuild_count(stream=stream) - r0
     own = bool(sol.get_option(api.SPH_OPT_INSTANCE_DECISIONS)) and hi - lo > 1
+    # lists shared by two particles (SPH_OPT_PARTICLES_PER_THREAD): a padded work order
+    padded = (hi - lo > 1 and not own and precision in ("fp32", "mixed_abs") and n >= 400000
+              and sol.get_option(api.SPH_OPT_PASS1_LANES) == 1
+              and sol.get_option(api.SPH_OPT_PARTICLES_PER_THREAD) == 1)
     out = {"value": n_all * steps / (ms / 1e3), "unit": UNIT,
            "fluid_value": n_fluid_all * steps / (ms / 1e3), "ms_per_step": ms / steps,
            "steps": steps, "warmup": warmup,
@@ -600,7 +606,7 @@ def batch_measure(n_inst: int, precision: str, args, stream, steps: int, warmup:
            "list_rebuilds": {"timed": rebuilds, "half_steps": 2 * steps},
            "gpu_launches": count_launches(
                sol_cells_batch(p, n_inst, skin, lanes["cell_divisions"]), 2 * steps,
-               rebuilds, args.graph_mode, own, particles=n),
+               rebuilds, args.graph_mode, own, particles=n, padded=padded),
            "autotune": None}
     if tuned:
         from tmp_sph_gb300 import autotune
